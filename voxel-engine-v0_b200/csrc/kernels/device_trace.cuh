@@ -540,10 +540,32 @@ __device__ __forceinline__ GrassSegFrame grass_seg_frame(const GrassBladeGeom& B
   return f;
 }
 
-__device__ __forceinline__ float grass_seg_sdf(const GrassSegFrame& f, v3 p) {
+// The minimum over boxes of sdf_box(local) = outside + inside (grass.wgsl:
+// 106-111), kept as its two parts: outside = sqrt(|max(q, 0)|^2) is 0 where
+// inside < 0 and inside is 0 elsewhere, and the correctly rounded square root
+// is monotone, so the minimum is the least inside when that is negative and
+// the square root of the least |max(q, 0)|^2 otherwise -- the same bits with
+// one square root per evaluation instead of one per box (18 at lod 0).  The
+// marches are bound by instruction issue; with the six normal taps in one
+// pass (grass_sdf_normal_lod): 1080p frame 4.71 -> 4.57 ms, 256x144 frame
+// 0.69 -> 0.57 ms, the 64-request batch 93.3 -> 87.5 ms.
+struct SdfMin {
+  float ss, in;
+};
+__device__ __forceinline__ SdfMin sdf_min_init() { return SdfMin{__int_as_float(0x7F800000), 0.0f}; }
+__device__ __forceinline__ void sdf_min_box(SdfMin& m, v3 local, float half_w, float half_h) {
+  const v3 q = V3(fabsf(local.x) - half_w, fabsf(local.y) - half_h, fabsf(local.z) - half_w);
+  const v3 o = vmax(q, V3s(0.0f));
+  m.ss = fmin_(m.ss, dot(o, o));
+  m.in = fmin_(m.in, fmax_(q.x, fmax_(q.y, q.z)));
+}
+__device__ __forceinline__ float sdf_min_value(const SdfMin& m) {
+  return m.in < 0.0f ? m.in : fmin_(BIG, sqrtf(m.ss));
+}
+
+__device__ __forceinline__ void grass_seg_sdf(SdfMin& m, const GrassSegFrame& f, v3 p) {
   const v3 d = p - f.mid;
-  const v3 local = V3(dot(d, f.S), dot(d, f.T), dot(d, f.N));
-  return sdf_box(local, V3s(0.0f), V3(f.half_w, f.half_h, f.half_w));
+  sdf_min_box(m, V3(dot(d, f.S), dot(d, f.T), dot(d, f.N)), f.half_w, f.half_h);
 }
 
 // Blade length of cell `id` (grass.wgsl:216).
@@ -724,59 +746,106 @@ __device__ __noinline__ bool grass_frames_ready(const Scene& s, GrassCellGeom& G
   return true;
 }
 
-// grass_sdf_lod (grass.wgsl:192-350) over the cached cell geometry.
-__device__ __noinline__ float grass_sdf_cached(const Scene& s, v3 p, v3 cb, v3 id, float time_s, float strength,
-                                               uint32_t lod, GrassCellGeom& G) {
-  const float vs = vs_(s);
+// False when the point is outside the cell's grass layer, where grass_sdf_lod
+// is BIG (grass.wgsl:204-213).
+__device__ __forceinline__ bool grass_in_layer(v3 p, v3 cb, float vs) {
   const float top_y = cb.y + vs;
   const float layer_h = GRASS_LAYER_HEIGHT_VOX * vs;
   const float y01 = (p.y - top_y) / fmax_(layer_h, 1e-6f);
-  if (y01 < 0.0f || y01 > 1.0f) return BIG;
+  if (y01 < 0.0f || y01 > 1.0f) return false;
   const float over = GRASS_OVERHANG_VOX * vs;
-  if (p.x < cb.x - over || p.x > cb.x + vs + over || p.z < cb.z - over || p.z > cb.z + vs + over) return BIG;
+  return !(p.x < cb.x - over || p.x > cb.x + vs + over || p.z < cb.z - over || p.z > cb.z + vs + over);
+}
+
+// Segment k of the record's lod-0 frames (grass_frames_ready).
+__device__ __forceinline__ GrassSegFrame grass_frame_load(const float4* F, uint32_t k) {
+  const float4 a = F[3u * k], b = F[3u * k + 1u], c = F[3u * k + 2u];
+  GrassSegFrame f;
+  f.mid = V3(a.x, a.y, a.z);
+  f.S = V3(b.x, b.y, b.z);
+  f.T = V3(c.x, c.y, c.z);
+  f.N = cross(f.T, f.S);
+  f.half_w = a.w;
+  f.half_h = b.w;
+  return f;
+}
+
+// grass_sdf_lod (grass.wgsl:192-350) over the cached cell geometry.
+__device__ __noinline__ float grass_sdf_cached(const Scene& s, v3 p, v3 cb, v3 id, float time_s, float strength,
+                                               uint32_t lod, GrassCellGeom& G) {
+  if (!grass_in_layer(p, cb, vs_(s))) return BIG;
   if (!G.built) grass_cell_build(s, cb, id, time_s, strength, lod, G);
-  float dmin = BIG;
+  SdfMin m = sdf_min_init();
   if (G.frames == 1u || (G.frames == 0u && grass_frames_ready(s, G))) {
     const float4* F = s.grass_frames + G.rec * GRASS_FRAME_F4;
 #pragma unroll 6
-    for (uint32_t k = 0; k < GRASS_FRAME_SEGS; ++k) {
-      const float4 a = F[3u * k], b = F[3u * k + 1u], c = F[3u * k + 2u];
-      GrassSegFrame f;
-      f.mid = V3(a.x, a.y, a.z);
-      f.S = V3(b.x, b.y, b.z);
-      f.T = V3(c.x, c.y, c.z);
-      f.N = cross(f.T, f.S);
-      f.half_w = a.w;
-      f.half_h = b.w;
-      dmin = fmin_(dmin, grass_seg_sdf(f, p));
-    }
-    return dmin;
+    for (uint32_t k = 0; k < GRASS_FRAME_SEGS; ++k) grass_seg_sdf(m, grass_frame_load(F, k), p);
+  } else {
+    for (uint32_t i = 0; i < G.blade_count; ++i)
+      for (uint32_t sg = 0; sg < G.segs; ++sg)
+        grass_seg_sdf(m, grass_seg_frame(G.blade[i], G.blade_len, G.inv_segs, G.taper[sg], sg), p);
   }
-  for (uint32_t i = 0; i < G.blade_count; ++i)
-    for (uint32_t sg = 0; sg < G.segs; ++sg)
-      dmin = fmin_(dmin, grass_seg_sdf(grass_seg_frame(G.blade[i], G.blade_len, G.inv_segs, G.taper[sg], sg), p));
-  return dmin;
+  return sdf_min_value(m);
 }
 
+// One box against the six normal taps p +- e along x, y and z (in that
+// order).  A tap differs from p in one coordinate, so the products of the
+// other two are shared; every sum keeps dot()'s order ((x + y) + z).
+__device__ __forceinline__ void grass_seg_taps(SdfMin* m, const GrassSegFrame& f, v3 p, v3 pp, v3 pm) {
+  const v3 d = p - f.mid, dp = pp - f.mid, dm = pm - f.mid;
+  const v3 axis[3] = {f.S, f.T, f.N};
+  float l[6][3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    const v3 A = axis[a];
+    const float x = d.x * A.x, y = d.y * A.y, z = d.z * A.z, xy = x + y;
+    l[0][a] = (dp.x * A.x + y) + z;
+    l[1][a] = (dm.x * A.x + y) + z;
+    l[2][a] = (x + dp.y * A.y) + z;
+    l[3][a] = (x + dm.y * A.y) + z;
+    l[4][a] = xy + dp.z * A.z;
+    l[5][a] = xy + dm.z * A.z;
+  }
+#pragma unroll
+  for (int k = 0; k < 6; ++k) sdf_min_box(m[k], V3(l[k][0], l[k][1], l[k][2]), f.half_w, f.half_h);
+}
+
+// The lod-0 normal's six SDF taps in one pass over the cell's boxes: each
+// box frame is loaded (or derived) once for all six instead of once per tap.
 __device__ __noinline__ v3 grass_sdf_normal_lod(const Scene& s, v3 p, v3 cb, v3 id, float time_s, float strength,
                                                 uint32_t lod, GrassCellGeom& G) {
   // grass.wgsl:370-408
+  const float vs = vs_(s);
   if (lod != 0u) {
-    const float vs = vs_(s);
     const float top_y = cb.y + vs;
     const v3 root = V3(cb.x + 0.5f * vs, top_y, cb.z + 0.5f * vs);
     const v2 w = grass_wind_xz(root, time_s, strength);
     const float tilt = 0.35f;
     return normalize(V3(-w.x * tilt, 1.0f, -w.y * tilt));
   }
-  const float e = 0.01f * vs_(s);
-  const float dx = grass_sdf_cached(s, p + V3(e, 0.0f, 0.0f), cb, id, time_s, strength, lod, G) -
-                   grass_sdf_cached(s, p - V3(e, 0.0f, 0.0f), cb, id, time_s, strength, lod, G);
-  const float dy = grass_sdf_cached(s, p + V3(0.0f, e, 0.0f), cb, id, time_s, strength, lod, G) -
-                   grass_sdf_cached(s, p - V3(0.0f, e, 0.0f), cb, id, time_s, strength, lod, G);
-  const float dz = grass_sdf_cached(s, p + V3(0.0f, 0.0f, e), cb, id, time_s, strength, lod, G) -
-                   grass_sdf_cached(s, p - V3(0.0f, 0.0f, e), cb, id, time_s, strength, lod, G);
-  return normalize(V3(dx, dy, dz));
+  const float e = 0.01f * vs;
+  const v3 pp = p + V3s(e), pm = p - V3s(e);
+  const bool in[6] = {grass_in_layer(V3(pp.x, p.y, p.z), cb, vs), grass_in_layer(V3(pm.x, p.y, p.z), cb, vs),
+                      grass_in_layer(V3(p.x, pp.y, p.z), cb, vs), grass_in_layer(V3(p.x, pm.y, p.z), cb, vs),
+                      grass_in_layer(V3(p.x, p.y, pp.z), cb, vs), grass_in_layer(V3(p.x, p.y, pm.z), cb, vs)};
+  if (!G.built) grass_cell_build(s, cb, id, time_s, strength, lod, G);
+  SdfMin m[6];
+#pragma unroll
+  for (int k = 0; k < 6; ++k) m[k] = sdf_min_init();
+  if (G.frames == 1u || (G.frames == 0u && grass_frames_ready(s, G))) {
+    const float4* F = s.grass_frames + G.rec * GRASS_FRAME_F4;
+#pragma unroll 1
+    for (uint32_t k = 0; k < GRASS_FRAME_SEGS; ++k) grass_seg_taps(m, grass_frame_load(F, k), p, pp, pm);
+  } else {
+    for (uint32_t i = 0; i < G.blade_count; ++i)
+#pragma unroll 1
+      for (uint32_t sg = 0; sg < G.segs; ++sg)
+        grass_seg_taps(m, grass_seg_frame(G.blade[i], G.blade_len, G.inv_segs, G.taper[sg], sg), p, pp, pm);
+  }
+  float d[6];
+#pragma unroll
+  for (int k = 0; k < 6; ++k) d[k] = in[k] ? sdf_min_value(m[k]) : BIG;
+  return normalize(V3(d[0] - d[1], d[2] - d[3], d[4] - d[5]));
 }
 
 __device__ __noinline__ float grass_self_shadow(const Scene& s, v3 hp, v3 cb, v3 id, float time_s, float strength, uint32_t lod) {

@@ -848,21 +848,67 @@ __device__ __noinline__ v3 grass_sdf_normal_lod(const Scene& s, v3 p, v3 cb, v3 
   return normalize(V3(d[0] - d[1], d[2] - d[3], d[4] - d[5]));
 }
 
+// The six (lod 0) or four sun samples of grass_self_shadow do not depend on
+// one another's distances, so they are taken in one pass over the cell's
+// boxes: a box frame (about 150 instructions where the cell is not a table
+// record, which is the rule here) is derived once for all samples instead of
+// once per sample.  The sample points are stepped anew for every box, three
+// additions each, rather than held in registers.  1080p frame 4.57 -> 4.34 ms,
+// 256x144 frame 0.57 -> 0.52 ms.
+template <uint32_t N>
+__device__ __forceinline__ float grass_sun_occlusion(const Scene& s, v3 p0, v3 step, v3 cb, v3 id, float time_s,
+                                                     float strength, uint32_t lod) {
+  const float vs = vs_(s);
+  uint32_t in = 0u;
+  v3 p = p0;
+#pragma unroll
+  for (uint32_t i = 0; i < N; ++i) {
+    if (grass_in_layer(p, cb, vs)) in |= 1u << i;
+    p = p + step;
+  }
+  SdfMin m[N];
+#pragma unroll
+  for (uint32_t i = 0; i < N; ++i) m[i] = sdf_min_init();
+  if (in != 0u) {
+    GrassCellGeom G;
+    grass_cell_build(s, cb, id, time_s, strength, lod, G);
+    auto box = [&](const GrassSegFrame& f) {
+      v3 q = p0;
+#pragma unroll
+      for (uint32_t i = 0; i < N; ++i) {
+        grass_seg_sdf(m[i], f, q);
+        q = q + step;
+      }
+    };
+    if (G.frames == 0u && grass_frames_ready(s, G)) {
+      const float4* F = s.grass_frames + G.rec * GRASS_FRAME_F4;
+#pragma unroll 1
+      for (uint32_t k = 0; k < GRASS_FRAME_SEGS; ++k) box(grass_frame_load(F, k));
+    } else {
+      for (uint32_t b = 0; b < G.blade_count; ++b)
+#pragma unroll 1
+        for (uint32_t sg = 0; sg < G.segs; ++sg)
+          box(grass_seg_frame(G.blade[b], G.blade_len, G.inv_segs, G.taper[sg], sg));
+    }
+  }
+  float occ = 0.0f;
+#pragma unroll
+  for (uint32_t i = 0; i < N; ++i) {
+    const float d = (in >> i) & 1u ? sdf_min_value(m[i]) : BIG;
+    occ += clampf(1.0f - d / (0.05f * vs), 0.0f, 1.0f);
+  }
+  return occ;
+}
+
 __device__ __noinline__ float grass_self_shadow(const Scene& s, v3 hp, v3 cb, v3 id, float time_s, float strength, uint32_t lod) {
   // grass.wgsl:410-447
   const float vs = vs_(s);
-  GrassCellGeom G;
-  G.built = false;
-  v3 p = hp + SUN_DIR * (0.02f * vs);
+  const v3 p = hp + SUN_DIR * (0.02f * vs);
   const float max_dist = (0.55f + 0.35f * (float)lod) * vs;
   const uint32_t steps = lod != 0u ? 4u : 6u;
   const float dt = max_dist / (float)steps;
-  float occ = 0.0f;
-  for (uint32_t i = 0; i < steps; ++i) {
-    const float d = grass_sdf_cached(s, p, cb, id, time_s, strength, lod, G);
-    occ += clampf(1.0f - d / (0.05f * vs), 0.0f, 1.0f);
-    p = p + SUN_DIR * dt;
-  }
+  const float occ = lod != 0u ? grass_sun_occlusion<4>(s, p, SUN_DIR * dt, cb, id, time_s, strength, lod)
+                              : grass_sun_occlusion<6>(s, p, SUN_DIR * dt, cb, id, time_s, strength, lod);
   return expf_(-0.35f * occ);
 }
 

@@ -84,16 +84,19 @@ struct BatchArgs {
   float4* slab_res;
   uint32_t* slab_hits;
   uint32_t slab_cap;
+  uint32_t slab_bits;             // SlabSink::bits
   uint32_t ray_cap;               // per-ray arrays' capacity
   unsigned long long* px_first;
   uint32_t* px_task;
   uint2* px_mask;
   uint2* px_probe;
   uint4* px_hit;                  // 4 x uint4 per ray: voxel answer of a ray that met probes or needs refining
+  uint4* px_gov;                  // per pending ray: the blade march its walk left open (FrameArgs::px_gov)
   uint32_t* q_pending;
   uint32_t* q_refine;             // rays whose answer is a grass voxel (grass-slab refinement)
   uint32_t* q_far;                // rays without a voxel answer (heightfield)
-  uint32_t* dcount;               // [0] probes, [1] pending rays, [2] slab tasks, [3] slab hits, [4] refine, [5] far
+  uint32_t* dcount;               // [0] probes, [1] pending rays, [2] slab tasks, [3] slab hits, [4] refine, [5] far,
+                                  // [6] bin positions given out; from [16] the slab bins
   // coherent queries: query rays binned by (origin chunk, direction octant)
   uint32_t* q_keys;               // bin of each query ray
   uint32_t* q_perm;               // query rays in bin order
@@ -297,14 +300,16 @@ __device__ __forceinline__ void batch_item(const BatchArgs& B, const BatchHeader
         ph.recs = B.probe_recs;
         ph.rec_count = &B.dcount[0];
         ph.rec_cap = B.probe_cap;
+        ph.defer_gov = true;
       }
       const VoxTraceResult vt = viewport_trace<DEFER ? PROBE_RECORD : PROBE_INLINE>(s, B.tile_count + q.tile_base,
                                                B.tile_slots + (size_t)q.tile_base * TILE_CANDS, q.tiles_x, gx, gy, ph);
       const bool vox = vt.in_grid && vt.best.hit != 0u;
       if (!DEFER) {
         store_rec_at(q.out, (size_t)gy * q.w + gx, viewport_finish(s, gx, gy, vox, vt.best));
-      } else if (ph.seq != 0u) {  // met probes: k_batch_resolve decides
+      } else if (ph.seq != 0u || (vox && vt.gov_state != 0u)) {  // met probes or left a blade march open: k_batch_resolve decides
         if (vox) store_hitgeom(B.px_hit + (size_t)ray * 4u, vt.best);
+        B.px_gov[ray] = make_uint4(vox ? vt.gov_state : 0u, __float_as_uint(vt.gov_t0), __float_as_uint(vt.gov_t1), vt.gov_slot);
         const uint32_t stored = ph.seq > 0xFFFFFFu ? 0u : ph.recorded;
         B.px_probe[ray] = make_uint2(probe_summary(ph.seq, ph.best_cand, ph.phase, ph.first_phase == 0u, vox), stored);
         enqueue_active(B.q_pending, &B.dcount[1], ray);
@@ -419,8 +424,13 @@ __global__ void __launch_bounds__(BATCH_THREADS) k_batch_defer_clear(const __gri
   }
 }
 
+__device__ __forceinline__ SlabSink slab_sink(const BatchArgs& B) {
+  return SlabSink{reinterpret_cast<uint4*>(B.slab_res), B.slab_hits, &B.dcount[2], B.slab_cap, B.dcount + 16, B.slab_bits};
+}
+
 __global__ void __launch_bounds__(BATCH_THREADS) k_batch_probe_dda(const __grid_constant__ BatchArgs B) {
   const uint32_t n_reqs = B.hdr->n_reqs;
+  const SlabSink sink = slab_sink(B);
   const uint32_t n = min(B.dcount[0], B.probe_cap);
   for (uint32_t i = blockIdx.x * BATCH_THREADS + threadIdx.x; i < n; i += gridDim.x * BATCH_THREADS) {
     const ProbeRec r = B.probe_recs[i];
@@ -440,57 +450,117 @@ __global__ void __launch_bounds__(BATCH_THREADS) k_batch_probe_dda(const __grid_
                         // is no task
                         const v2 iv = grass_slab_interval(ro, rd, t, tNext, id * vs, vs);
                         if (iv.y <= iv.x) return false;
-                        const uint32_t j = atomicAdd(&B.dcount[2], 1u);
-                        if (j < B.slab_cap) {
-                          B.slab_tasks[j] = slab_task(i, it, iv.x, iv.y, id, ch);
-                        } else {
-                          lost = true;
-                        }
+                        lost |= !slab_push(sink, slab_task(i, it, iv.x, iv.y, id, ch, r.slot, 0u));
                         return false;
                       });
     if (lost) atomicMin(&B.px_probe[r.pixel].y, 0u);
   }
+  // the blade marches the walks left open
+  const uint32_t np = B.dcount[1];
+  for (uint32_t i = blockIdx.x * BATCH_THREADS + threadIdx.x; i < np; i += gridDim.x * BATCH_THREADS) {
+    const uint32_t ray = B.q_pending[i];
+    const uint4 gv = B.px_gov[ray];
+    if (gv.x != 1u) continue;
+    const BatchRay br = batch_ray(B, n_reqs, ray);
+    const Scene s = batch_scene(B, &B.cams[br.q->cam]);
+    const uint4 h = B.px_hit[(size_t)ray * 4u];
+    if (!slab_push(sink, slab_gov_task(s, ray, gv.w, cam_pos(s),
+                                       ray_dir_from_pixel(s, V2((float)br.gx + 0.5f, (float)br.gy + 0.5f)),
+                                       __uint_as_float(h.x),
+                                       V3(__uint_as_float(h.y), __uint_as_float(h.z), __uint_as_float(h.w)),
+                                       __uint_as_float(gv.y), __uint_as_float(gv.z))))
+      B.px_gov[ray].x = 2u;
+  }
+}
+
+__global__ void __launch_bounds__(BATCH_THREADS) k_batch_slab_bases(const __grid_constant__ BatchArgs B) {
+  slab_bases(slab_sink(B), &B.dcount[6]);
+}
+__global__ void __launch_bounds__(BATCH_THREADS) k_batch_slab_order(const __grid_constant__ BatchArgs B) {
+  slab_order(slab_sink(B), B.slab_tasks);
+}
+
+// A slab task with its ray and its cell.
+struct BatchSlab {
+  uint4 a;
+  bool gov;
+  uint32_t ray, slot;
+  Scene s;
+  v3 ro, rd, id, cb;
+};
+__device__ __forceinline__ BatchSlab batch_slab(const BatchArgs& B, uint32_t n_reqs, uint32_t j) {
+  BatchSlab w;
+  w.a = B.slab_tasks[j];
+  w.gov = (w.a.y & SLAB_GOV) != 0u;
+  if (w.gov) {
+    w.ray = w.a.x;
+    w.slot = B.px_gov[w.ray].w;
+  } else {
+    const uint4 r = *reinterpret_cast<const uint4*>(&B.probe_recs[w.a.x]);
+    w.ray = r.x;
+    w.slot = r.y;
+  }
+  const BatchRay br = batch_ray(B, n_reqs, w.ray);
+  w.s = batch_scene(B, &B.cams[br.q->cam]);
+  w.ro = cam_pos(w.s);
+  w.rd = ray_dir_from_pixel(w.s, V2((float)br.gx + 0.5f, (float)br.gy + 0.5f));
+  const Meta ch = meta_at(w.s, w.slot);
+  w.id = slab_task_cell(w.a, ch);
+  w.cb = slab_task_corner(w.a, ch, w.id, vs_(w.s));
+  return w;
 }
 
 __global__ void __launch_bounds__(BATCH_THREADS, SLAB_MIN_BLOCKS) k_batch_slab_eval(const __grid_constant__ BatchArgs B) {
   const uint32_t n_reqs = B.hdr->n_reqs;
   const uint32_t n = min(B.dcount[2], B.slab_cap);
   for (uint32_t j = blockIdx.x * BATCH_THREADS + threadIdx.x; j < n; j += gridDim.x * BATCH_THREADS) {
-    const uint4 a = B.slab_tasks[j];
-    const ProbeRec r = B.probe_recs[a.x];
-    const BatchRay br = batch_ray(B, n_reqs, r.pixel);
-    const Scene s = batch_scene(B, &B.cams[br.q->cam]);
-    const float vs = vs_(s);
-    const v3 ro = cam_pos(s);
-    const v3 rd = ray_dir_from_pixel(s, V2((float)br.gx + 0.5f, (float)br.gy + 0.5f));
-    const v3 id = slab_task_cell(a, meta_at(s, r.slot));
-    const float t0 = __uint_as_float(a.z);  // the slab interval (non-empty)
-    const GrassHit gh = grass_layer_trace_lod(s, ro, rd, t0, __uint_as_float(a.w), id * vs, id, s.cam->voxel_params[1],
-                                              s.cam->voxel_params[2], grass_lod_from_t(t0));
-    if (gh.hit) {
-      if (__float_as_uint(gh.t) & 0x80000000u) {
-        atomicMin(&B.px_probe[r.pixel].y, 0u);
+    const BatchSlab w = batch_slab(B, n_reqs, j);
+    float t;
+    if (!slab_march(w.s, w.ro, w.rd, w.a, w.slot, w.cb, w.id, &t)) {
+      if (w.gov) B.px_gov[w.ray].x = 4u;  // the voxel hit stands
+      continue;
+    }
+    B.slab_res[j].x = t;
+    if (!w.gov) {
+      if (__float_as_uint(t) & 0x80000000u) {
+        atomicMin(&B.px_probe[w.ray].y, 0u);
         continue;
       }
+      const ProbeRec r = B.probe_recs[w.a.x];
       const uint32_t cand = probe_cand(r), phase = probe_phase(r);
-      B.slab_res[j] = make_float4(gh.t, gh.n.x, gh.n.y, gh.n.z);
-      atomicMin(&B.px_first[r.pixel], slab_key(phase, gh.t, cand, probe_seq(r), slab_task_step(a)));
-      atomicOr(phase ? &B.px_mask[r.pixel].y : &B.px_mask[r.pixel].x, 1u << (cand & 31u));
-      B.slab_hits[atomicAdd(&B.dcount[3], 1u)] = j;
+      atomicMin(&B.px_first[w.ray], slab_key(phase, t, cand, probe_seq(r), slab_task_step(w.a)));
+      atomicOr(phase ? &B.px_mask[w.ray].y : &B.px_mask[w.ray].x, 1u << (cand & 31u));
     }
+    B.slab_hits[atomicAdd(&B.dcount[3], 1u)] = j;
   }
 }
 
 __global__ void __launch_bounds__(BATCH_THREADS) k_batch_slab_pick(const __grid_constant__ BatchArgs B) {
+  const uint32_t n_reqs = B.hdr->n_reqs;
   const uint32_t n = min(B.dcount[3], B.slab_cap);
   for (uint32_t i = blockIdx.x * BATCH_THREADS + threadIdx.x; i < n; i += gridDim.x * BATCH_THREADS) {
     const uint32_t j = B.slab_hits[i];
     const uint4 a = B.slab_tasks[j];
-    const ProbeRec r = B.probe_recs[a.x];
-    const unsigned long long key = slab_key(probe_phase(r), B.slab_res[j].x, probe_cand(r), probe_seq(r), slab_task_step(a));
-    const unsigned long long first = B.px_first[r.pixel];
-    if (key == first) B.px_task[r.pixel] = j;
-    else if (slab_hit_shadows_first(first, key)) atomicMin(&B.px_probe[r.pixel].y, 0u);
+    const float t = B.slab_res[j].x;
+    if ((a.y & SLAB_GOV) == 0u) {
+      const ProbeRec r = B.probe_recs[a.x];
+      const unsigned long long key = slab_key(probe_phase(r), t, probe_cand(r), probe_seq(r), slab_task_step(a));
+      const unsigned long long first = B.px_first[r.pixel];
+      if (key != first) {
+        if (slab_hit_shadows_first(first, key)) atomicMin(&B.px_probe[r.pixel].y, 0u);
+        continue;
+      }
+    }
+    const BatchSlab w = batch_slab(B, n_reqs, j);
+    const v3 nrm = slab_normal(w.s, w.ro, w.rd, w.a, w.slot, w.cb, w.id, t);
+    if (w.gov) {
+      B.px_hit[(size_t)w.ray * 4u] =
+          make_uint4(__float_as_uint(t), __float_as_uint(nrm.x), __float_as_uint(nrm.y), __float_as_uint(nrm.z));
+      B.px_gov[w.ray].x = 3u;
+    } else {
+      B.slab_res[j] = make_float4(t, nrm.x, nrm.y, nrm.z);
+      B.px_task[w.ray] = j;
+    }
   }
 }
 
@@ -509,7 +579,8 @@ __global__ void __launch_bounds__(BATCH_THREADS) k_batch_resolve(const __grid_co
     const BatchRay br = batch_ray(B, n_reqs, ray);
     const BatchReq& q = *br.q;
     const Scene s = batch_scene(B, &B.cams[q.cam]);
-    bool walk = pp.y < met;
+    // some probes were not evaluated, or a march left open could change which chunk answers
+    bool walk = pp.y < met || B.px_gov[ray].x == 2u;
     if (!walk && first != ~0ull) {
       const uint32_t j = B.px_task[ray];
       const float4 res = B.slab_res[j];

@@ -62,7 +62,8 @@ struct FrameArgs {
   uint32_t* q_vox;    // pixel ids with a voxel hit
   uint32_t* q_far;    // pixel ids for heightfield / sky
   uint32_t* q_count;  // [0] voxel, [1] far, [2] fresh shadow, [3] light gather, [4] probes, [5] pending,
-                      // [6] slab tasks, [7] slab hits, [8] far pixels queued by the walk
+                      // [6] slab tasks, [7] slab hits, [8] far pixels queued by the walk, [11] bin positions
+                      // given out, [12] / [13] the gov tasks / hits among [6] / [7]; then the slab bins
   uint32_t* q_shadow;  // voxel pixels that trace a fresh sun shadow this frame
   uint32_t* q_light;   // voxel pixels that gather local lights
   float* px_shadow;    // fresh sun transmittance per pixel (q_shadow pixels)
@@ -71,16 +72,17 @@ struct FrameArgs {
   // -> k_slab_pick -> k_primary_resolve)
   ProbeRec* probe_recs;           // stored probes, q_count[4] of them (capped)
   uint32_t probe_cap;
-  uint4* slab_tasks;              // one uint4 (slab_task) per grass column slab to march, q_count[6] of them
-  float4* slab_res;               // per slab task: hit t, normal (written on hits)
-  uint32_t* slab_hits;            // slab tasks that hit, q_count[7] of them
+  uint4* slab_tasks;              // one uint4 (slab_task) per grass slab to march, q_count[6] of them, sorted
+  float4* slab_res;               // the tasks as found; once sorted, per task: hit t, the pixel's nearest hit's normal
+  uint32_t* slab_hits;            // per task as found: rank in its bin; once sorted, the tasks that hit (q_count[7])
   uint32_t slab_cap;
+  uint32_t slab_bits;             // SlabSink::bits
   unsigned long long* px_first;   // per pixel: nearest probe hit key (slab_key), ~0 = none
   uint32_t* px_task;              // per pixel: the slab task with that key
   uint2* px_mask;                 // per pixel: candidate chunks with a probe hit, hint / full trace
   uint2* px_probe;                // per pixel: walk summary (probe_summary) | probes stored
   uint4* px_gov = nullptr;        // per pending pixel: deferred blade march of its answer (gov_state,
-                                  // interval, chunk slot); 3 / 4 once k_gov_eval ran it (hit / miss)
+                                  // interval, chunk slot); 3 / 4 once k_slab_pick / k_slab_eval ran it (hit / miss)
   uint32_t* q_pending;            // pixels whose walk met probes, q_count[5] of them
   // per-frame grass cell table: written by k_grass_cells, read by the rest
   float4* grass_rec;
@@ -951,8 +953,12 @@ __global__ void __launch_bounds__(PRIMARY_THREADS) k_primary_trace_views(const _
 // One lane per stored probe: the probe's column DDA with the walk's
 // arguments, storing one task per grass slab it would march.  A probe whose
 // tasks do not all fit sends its pixel to the inline walk (stored count 0).
+__device__ __forceinline__ SlabSink slab_sink(const FrameArgs& A) {
+  return SlabSink{reinterpret_cast<uint4*>(A.slab_res), A.slab_hits, &A.q_count[6], A.slab_cap, A.q_count + 16, A.slab_bits};
+}
 __device__ __forceinline__ void k_probe_dda_body(const FrameArgs& A) {
   const Scene s = make_scene(A, false);
+  const SlabSink sink = slab_sink(A);
   const uint32_t n = min(A.q_count[4], A.probe_cap);
   const float vs = vs_(s);
   for (uint32_t i = blockIdx.x * SHADE_THREADS + threadIdx.x; i < n; i += gridDim.x * SHADE_THREADS) {
@@ -969,15 +975,25 @@ __device__ __forceinline__ void k_probe_dda_body(const FrameArgs& A) {
                         // is no task
                         const v2 iv = grass_slab_interval(c.ro, c.rd, t, tNext, id * vs, vs);
                         if (iv.y <= iv.x) return false;
-                        const uint32_t j = atomicAdd(&A.q_count[6], 1u);
-                        if (j < A.slab_cap) {
-                          A.slab_tasks[j] = slab_task(i, it, iv.x, iv.y, id, ch);
-                        } else {
-                          lost = true;
-                        }
+                        lost |= !slab_push(sink, slab_task(i, it, iv.x, iv.y, id, ch, r.slot, 0u));
                         return false;
                       });
     if (lost) atomicMin(&A.px_probe[r.pixel].y, 0u);
+  }
+  // the blade marches the walk left open are tasks too; one that does not fit
+  // leaves its pixel's voxel answer undecided
+  const uint32_t np = A.px_gov ? A.q_count[5] : 0u;
+  for (uint32_t i = blockIdx.x * SHADE_THREADS + threadIdx.x; i < np; i += gridDim.x * SHADE_THREADS) {
+    const uint32_t pix = A.q_pending[i];
+    const uint4 gv = A.px_gov[pix];
+    if (gv.x != 1u) continue;
+    const uint4 h = A.pix_hit[(size_t)pix * 5u];
+    const PrimaryCtx c = primary_ctx(s, pix % A.iw, pix / A.iw, A.iw);
+    atomicAdd(&A.q_count[12], 1u);
+    if (!slab_push(sink, slab_gov_task(s, pix, gv.w, c.ro, c.rd, __uint_as_float(h.x),
+                                       V3(__uint_as_float(h.y), __uint_as_float(h.z), __uint_as_float(h.w)),
+                                       __uint_as_float(gv.y), __uint_as_float(gv.z))))
+      A.px_gov[pix].x = 2u;
   }
 }
 __global__ void __launch_bounds__(SHADE_THREADS) k_probe_dda(const __grid_constant__ FrameArgs A) { k_probe_dda_body(A); }
@@ -985,32 +1001,73 @@ __global__ void __launch_bounds__(SHADE_THREADS) k_probe_dda_views(const __grid_
   k_probe_dda_body(V.v[blockIdx.z]);
 }
 
-// One lane per grass slab: try_grass_slab_hit (the blade march).  A hit
-// lowers its pixel's nearest-hit key and marks its chunk.
+// The sort of the slab tasks (SlabSink).
+__device__ __forceinline__ void k_slab_bases_body(const FrameArgs& A) { slab_bases(slab_sink(A), &A.q_count[11]); }
+__global__ void __launch_bounds__(SHADE_THREADS) k_slab_bases(const __grid_constant__ FrameArgs A) { k_slab_bases_body(A); }
+__global__ void __launch_bounds__(SHADE_THREADS) k_slab_bases_views(const __grid_constant__ FrameArgsViews V) {
+  k_slab_bases_body(V.v[blockIdx.z]);
+}
+__device__ __forceinline__ void k_slab_order_body(const FrameArgs& A) { slab_order(slab_sink(A), A.slab_tasks); }
+__global__ void __launch_bounds__(SHADE_THREADS) k_slab_order(const __grid_constant__ FrameArgs A) { k_slab_order_body(A); }
+__global__ void __launch_bounds__(SHADE_THREADS) k_slab_order_views(const __grid_constant__ FrameArgsViews V) {
+  k_slab_order_body(V.v[blockIdx.z]);
+}
+
+// A slab task with its pixel's ray and its cell.
+struct SlabWork {
+  uint4 a;
+  bool gov;
+  uint32_t pix, slot;
+  PrimaryCtx c;
+  v3 id, cb;
+};
+__device__ __forceinline__ SlabWork slab_work(const Scene& s, const FrameArgs& A, uint32_t j) {
+  SlabWork w;
+  w.a = A.slab_tasks[j];
+  w.gov = (w.a.y & SLAB_GOV) != 0u;
+  if (w.gov) {
+    w.pix = w.a.x;
+    w.slot = A.px_gov[w.pix].w;
+  } else {
+    const uint4 r = *reinterpret_cast<const uint4*>(&A.probe_recs[w.a.x]);
+    w.pix = r.x;
+    w.slot = r.y;
+  }
+  w.c = primary_ctx(s, w.pix % A.iw, w.pix / A.iw, A.iw);
+  const Meta ch = meta_at(s, w.slot);
+  w.id = slab_task_cell(w.a, ch);
+  w.cb = slab_task_corner(w.a, ch, w.id, vs_(s));
+  return w;
+}
+
+// One lane per grass slab: the blade march of try_grass_slab_hit.  A hit
+// lowers its pixel's nearest-hit key and marks its chunk; k_slab_pick takes
+// the normals, of the nearest hits only (13 % of the marches hit, and their
+// normals inside this kernel cost every warp about two more marches).
 __device__ __forceinline__ void k_slab_eval_body(const FrameArgs& A) {
   const Scene s = make_scene(A, false);
   const uint32_t n = min(A.q_count[6], A.slab_cap);
-  const float vs = vs_(s);
-  const float time_s = s.cam->voxel_params[1], strength = s.cam->voxel_params[2];
   for (uint32_t j = blockIdx.x * SHADE_THREADS + threadIdx.x; j < n; j += gridDim.x * SHADE_THREADS) {
-    const uint4 a = A.slab_tasks[j];
-    const ProbeRec r = A.probe_recs[a.x];
-    const PrimaryCtx c = primary_ctx(s, r.pixel % A.iw, r.pixel / A.iw, A.iw);
-    const v3 id = slab_task_cell(a, meta_at(s, r.slot));
-    const float t0 = __uint_as_float(a.z);  // the slab interval (non-empty)
-    const GrassHit gh = grass_layer_trace_lod(s, c.ro, c.rd, t0, __uint_as_float(a.w), id * vs, id, time_s, strength,
-                                              grass_lod_from_t(t0));
-    if (gh.hit) {
-      if (__float_as_uint(gh.t) & 0x80000000u) {  // not ordered by the key: walk again
-        atomicMin(&A.px_probe[r.pixel].y, 0u);
+    const SlabWork w = slab_work(s, A, j);
+    float t;
+    if (!slab_march(s, w.c.ro, w.c.rd, w.a, w.slot, w.cb, w.id, &t)) {
+      if (w.gov) A.px_gov[w.pix].x = 4u;  // the voxel hit stands
+      continue;
+    }
+    A.slab_res[j].x = t;
+    if (!w.gov) {
+      if (__float_as_uint(t) & 0x80000000u) {  // not ordered by the key: walk again
+        atomicMin(&A.px_probe[w.pix].y, 0u);
         continue;
       }
+      const ProbeRec r = A.probe_recs[w.a.x];
       const uint32_t cand = probe_cand(r), phase = probe_phase(r);
-      A.slab_res[j] = make_float4(gh.t, gh.n.x, gh.n.y, gh.n.z);
-      atomicMin(&A.px_first[r.pixel], slab_key(phase, gh.t, cand, probe_seq(r), slab_task_step(a)));
-      atomicOr(phase ? &A.px_mask[r.pixel].y : &A.px_mask[r.pixel].x, 1u << (cand & 31u));
-      A.slab_hits[atomicAdd(&A.q_count[7], 1u)] = j;
+      atomicMin(&A.px_first[w.pix], slab_key(phase, t, cand, probe_seq(r), slab_task_step(w.a)));
+      atomicOr(phase ? &A.px_mask[w.pix].y : &A.px_mask[w.pix].x, 1u << (cand & 31u));
+    } else {
+      atomicAdd(&A.q_count[13], 1u);
     }
+    A.slab_hits[atomicAdd(&A.q_count[7], 1u)] = j;
   }
 }
 __global__ void __launch_bounds__(SHADE_THREADS, SLAB_MIN_BLOCKS) k_slab_eval(const __grid_constant__ FrameArgs A) { k_slab_eval_body(A); }
@@ -1029,55 +1086,41 @@ __device__ __forceinline__ bool slab_hit_shadows_first(unsigned long long first,
   return first != ~0ull && (key & chunk_mask) == (first & chunk_mask) && (key & seq_mask) < (first & seq_mask);
 }
 
-// Finds, per pixel, the slab task whose key is the pixel's nearest; pixels
-// where that hit is not its chunk's first are sent to the inline walk.
+// Finds, per pixel, the slab task whose key is the pixel's nearest, and takes
+// its normal; pixels where that hit is not its chunk's first are sent to the
+// inline walk.  A hit of a march the walk left open replaces the answer's t
+// and n in its PixHit record.
 __device__ __forceinline__ void k_slab_pick_body(const FrameArgs& A) {
+  const Scene s = make_scene(A, false);
   const uint32_t n = min(A.q_count[7], A.slab_cap);
   for (uint32_t i = blockIdx.x * SHADE_THREADS + threadIdx.x; i < n; i += gridDim.x * SHADE_THREADS) {
     const uint32_t j = A.slab_hits[i];
     const uint4 a = A.slab_tasks[j];
-    const ProbeRec r = A.probe_recs[a.x];
-    const unsigned long long key =
-        slab_key(probe_phase(r), A.slab_res[j].x, probe_cand(r), probe_seq(r), slab_task_step(a));
-    const unsigned long long first = A.px_first[r.pixel];
-    if (key == first) A.px_task[r.pixel] = j;
-    else if (slab_hit_shadows_first(first, key)) atomicMin(&A.px_probe[r.pixel].y, 0u);
+    const float t = A.slab_res[j].x;
+    if ((a.y & SLAB_GOV) == 0u) {
+      const ProbeRec r = A.probe_recs[a.x];
+      const unsigned long long key = slab_key(probe_phase(r), t, probe_cand(r), probe_seq(r), slab_task_step(a));
+      const unsigned long long first = A.px_first[r.pixel];
+      if (key != first) {
+        if (slab_hit_shadows_first(first, key)) atomicMin(&A.px_probe[r.pixel].y, 0u);
+        continue;
+      }
+    }
+    const SlabWork w = slab_work(s, A, j);
+    const v3 nrm = slab_normal(s, w.c.ro, w.c.rd, w.a, w.slot, w.cb, w.id, t);
+    if (w.gov) {
+      A.pix_hit[(size_t)w.pix * 5u] =
+          make_uint4(__float_as_uint(t), __float_as_uint(nrm.x), __float_as_uint(nrm.y), __float_as_uint(nrm.z));
+      A.px_gov[w.pix].x = 3u;
+    } else {
+      A.slab_res[j] = make_float4(t, nrm.x, nrm.y, nrm.z);
+      A.px_task[w.pix] = j;
+    }
   }
 }
 __global__ void __launch_bounds__(SHADE_THREADS) k_slab_pick(const __grid_constant__ FrameArgs A) { k_slab_pick_body(A); }
 __global__ void __launch_bounds__(SHADE_THREADS) k_slab_pick_views(const __grid_constant__ FrameArgsViews V) {
   k_slab_pick_body(V.v[blockIdx.z]);
-}
-
-// The blade marches the walk deferred (grass_on_voxel_hit of a grass-voxel
-// answer, px_gov state 1), one lane per pending pixel: a hit replaces the
-// answer's t and n in its PixHit record (state 3), a miss keeps the voxel
-// hit (state 4).
-__device__ __forceinline__ void k_gov_eval_body(const FrameArgs& A) {
-  if (A.px_gov == nullptr) return;
-  const Scene s = make_scene(A, false);
-  const uint32_t n = A.q_count[5];
-  for (uint32_t i = blockIdx.x * SHADE_THREADS + threadIdx.x; i < n; i += gridDim.x * SHADE_THREADS) {
-    const uint32_t pix = A.q_pending[i];
-    const uint4 gv = A.px_gov[pix];
-    if (gv.x != 1u) continue;
-    uint4* rec = A.pix_hit + (size_t)pix * 5u;
-    const uint4 h0 = rec[0];
-    const PrimaryCtx c = primary_ctx(s, pix % A.iw, pix / A.iw, A.iw);
-    const GrassHit gh = grass_on_voxel_hit(s, c.ro, c.rd, meta_at(s, gv.w), __uint_as_float(h0.x),
-                                           V3(__uint_as_float(h0.y), __uint_as_float(h0.z), __uint_as_float(h0.w)),
-                                           __uint_as_float(gv.y), __uint_as_float(gv.z));
-    if (gh.hit)
-      rec[0] = make_uint4(__float_as_uint(gh.t), __float_as_uint(gh.n.x), __float_as_uint(gh.n.y),
-                          __float_as_uint(gh.n.z));
-    A.px_gov[pix].x = gh.hit ? 3u : 4u;
-  }
-}
-__global__ void __launch_bounds__(SHADE_THREADS, SLAB_MIN_BLOCKS) k_gov_eval(const __grid_constant__ FrameArgs A) {
-  k_gov_eval_body(A);
-}
-__global__ void __launch_bounds__(SHADE_THREADS, SLAB_MIN_BLOCKS) k_gov_eval_views(const __grid_constant__ FrameArgsViews V) {
-  k_gov_eval_body(V.v[blockIdx.z]);
 }
 
 // Pixels that met probes: the nearer of the nearest probe hit and the voxel

@@ -110,7 +110,7 @@ struct BatchLane {
   DevBuf hdr, reqs, cams, tile_count, tile_slots, head;
   // deferred grass probes of viewport rays: per-ray arrays for ray_cap rays,
   // probe records and slab tasks in proportion, counters
-  DevBuf probe_recs, slab_tasks, slab_res, slab_hits, px_first, px_task, px_mask, px_probe, px_hit, q_pending,
+  DevBuf probe_recs, slab_tasks, slab_res, slab_hits, px_first, px_task, px_mask, px_probe, px_hit, px_gov, q_pending,
       q_refine, q_far, dcount;
   uint32_t ray_cap = 0;
   // coherent queries: bin of each query ray, rays in bin order, bin counters
@@ -275,8 +275,13 @@ vxe_status alloc_on(vxe_ctx* c, DevBuf& b, size_t bytes, cudaStream_t st) {
 // Stored grass column probes per internal pixel (the walk meets about four
 // per pixel on grassland; pixels past the cap replay their walk).
 constexpr size_t kProbesPerPixel = 8;
+// Slab bins of a frame (SlabSink::bits): one chunk in 16 shares a lod-0 bin;
+// a view's lod-0 range (18 m, 60 degrees) crosses about that many.
+constexpr uint32_t kFrameSlabBits = 4;
 // Grass slab marches those probes ask for, per internal pixel.
 constexpr size_t kSlabsPerPixel = 4;
+
+constexpr size_t kQcountBytes = 64 + (size_t)(4096u << (kFrameSlabBits + 1u)) * 4;  // queue counters, then the slab bins
 
 size_t img_bytes(const FrameState& F, int i) {
   const size_t in = (size_t)F.iw * F.ih, pn = (size_t)F.pw * F.ph;
@@ -314,7 +319,7 @@ size_t img_bytes(const FrameState& F, int i) {
     case IMG_PXLIGHT: case IMG_GODPRE: case IMG_PXGOV:
       return in * 16;
     case IMG_QCOUNT:
-      return 64;
+      return kQcountBytes;
     default:
       return 0;
   }
@@ -584,12 +589,13 @@ void frame_fill(vxe_ctx* c, FrameState& F, const vxe_camera_gpu& cam, FrameArgs&
   A.slab_res = (float4*)S->img[IMG_SLAB_RES].p;
   A.slab_cap = (uint32_t)std::min<size_t>(S->img[IMG_SLAB_TASKS].bytes / 16u, 0xFFFFFFFFu);
   if (c->slab_limit) A.slab_cap = std::min(A.slab_cap, c->slab_limit);
+  A.slab_bits = kFrameSlabBits;
   A.px_first = (unsigned long long*)S->img[IMG_PXFIRST].p;
   A.px_probe = (uint2*)S->img[IMG_PXPROBE].p;
   A.slab_hits = (uint32_t*)S->img[IMG_SLAB_HITS].p;
   A.px_task = (uint32_t*)S->img[IMG_PXTASK].p;
   A.px_mask = (uint2*)S->img[IMG_PXMASK].p;
-  // the wavefront walk leaves grass-voxel blade marches to k_gov_eval
+  // the wavefront walk leaves grass-voxel blade marches to k_slab_eval
   A.px_gov = (c->flags & VXE_FLAG_PRIMARY_MEGAKERNEL) ? nullptr : (uint4*)S->img[IMG_PXGOV].p;
   A.q_pending = (uint32_t*)S->img[IMG_QPENDING].p;
   A.god_pre = (c->flags & VXE_FLAG_PRIMARY_MEGAKERNEL) ? nullptr : (float4*)S->img[IMG_GODPRE].p;
@@ -634,7 +640,7 @@ vxe_status frame_enqueue(vxe_ctx* c, FrameState& F, const FrameArgs& A, bool tim
       return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((threads + SHADE_THREADS - 1) / SHADE_THREADS,
                                                                 (uint64_t)c->shade_wave));
     };
-    CK(cudaMemsetAsync(A.q_count, 0, 64, st));
+    CK(cudaMemsetAsync(A.q_count, 0, kQcountBytes, st));
     vxe_status sr;
     if (side && (sr = side_ready(c, *side)) != VXE_OK) return sr;
     CK(cudaMemsetAsync(A.px_first, 0xFF, (size_t)npix * 8u, st));
@@ -652,10 +658,11 @@ vxe_status frame_enqueue(vxe_ctx* c, FrameState& F, const FrameArgs& A, bool tim
       k_godray_far<<<grid(npix), SHADE_THREADS, 0, side->s>>>(A);
     }
     k_probe_dda<<<grid((uint64_t)npix * kProbesPerPixel), SHADE_THREADS, 0, st>>>(A);
+    k_slab_bases<<<grid(slab_bins(kFrameSlabBits)), SHADE_THREADS, 0, st>>>(A);
+    k_slab_order<<<grid((uint64_t)npix * kSlabsPerPixel), SHADE_THREADS, 0, st>>>(A);
     if (F.table_wait) CK(cudaStreamWaitEvent(st, F.table_wait, 0));
     k_slab_eval<<<grid((uint64_t)npix * kSlabsPerPixel), SHADE_THREADS, 0, st>>>(A);
     k_slab_pick<<<grid(npix), SHADE_THREADS, 0, st>>>(A);
-    k_gov_eval<<<grid(npix), SHADE_THREADS, 0, st>>>(A);
     k_primary_resolve<<<grid(npix), SHADE_THREADS, 0, st>>>(A);
     if (timed) CK(cudaEventRecord(F.ev[3], st));
     if (side) {  // the far pixels the resolve queued, beside the voxel shading
@@ -714,7 +721,7 @@ vxe_status views_enqueue(vxe_ctx* c, const vxe::dev::FrameArgsViews& V, uint32_t
   for (uint32_t i = 0; i < n; ++i) {
     const FrameArgs& A = V.v[i];
     const size_t npix = (size_t)A.iw * A.ih;
-    CK(cudaMemsetAsync(A.q_count, 0, 64, st));
+    CK(cudaMemsetAsync(A.q_count, 0, kQcountBytes, st));
     CK(cudaMemsetAsync(A.px_first, 0xFF, npix * 8u, st));
     CK(cudaMemsetAsync(A.px_mask, 0, npix * 8u, st));
     if (A.god_pre) CK(cudaMemsetAsync(A.god_pre, 0, npix * 16u, st));
@@ -730,9 +737,10 @@ vxe_status views_enqueue(vxe_ctx* c, const vxe::dev::FrameArgsViews& V, uint32_t
   k_shade_far_views<0><<<grid(max_pix), SHADE_THREADS, 0, side->s>>>(V);
   k_godray_far_views<<<grid(max_pix), SHADE_THREADS, 0, side->s>>>(V);
   k_probe_dda_views<<<grid(max_pix * kProbesPerPixel), SHADE_THREADS, 0, st>>>(V);
+  k_slab_bases_views<<<grid(slab_bins(kFrameSlabBits)), SHADE_THREADS, 0, st>>>(V);
+  k_slab_order_views<<<grid(max_pix * kSlabsPerPixel), SHADE_THREADS, 0, st>>>(V);
   k_slab_eval_views<<<grid(max_pix * kSlabsPerPixel), SHADE_THREADS, 0, st>>>(V);
   k_slab_pick_views<<<grid(max_pix), SHADE_THREADS, 0, st>>>(V);
-  k_gov_eval_views<<<grid(max_pix), SHADE_THREADS, 0, st>>>(V);
   k_primary_resolve_views<<<grid(max_pix), SHADE_THREADS, 0, st>>>(V);
   CK(cudaEventRecord(side->mid, st));
   CK(cudaStreamWaitEvent(side->s, side->mid, 0));
@@ -1002,7 +1010,7 @@ void vxe_destroy(vxe_ctx* c) {
   for (auto& L : c->lanes) {
     if (L.stream) cudaStreamSynchronize(L.stream);
     for (auto* b : {&L.hdr, &L.reqs, &L.cams, &L.tile_count, &L.tile_slots, &L.head, &L.probe_recs, &L.slab_tasks,
-                    &L.slab_res, &L.slab_hits, &L.px_first, &L.px_task, &L.px_mask, &L.px_probe, &L.px_hit,
+                    &L.slab_res, &L.slab_hits, &L.px_first, &L.px_task, &L.px_mask, &L.px_probe, &L.px_hit, &L.px_gov,
                     &L.q_pending, &L.q_refine, &L.q_far, &L.dcount, &L.q_keys, &L.q_perm, &L.bin_count})
       release(*b, L.stream);
     release_frame_state(L.scratch, L.stream);
@@ -1549,8 +1557,8 @@ vxe_status vxe_get_frame_stats(vxe_ctx* c, vxe_frame_stats* out) {
   out->far_pixels = q[1];
   out->probes = q[4];
   out->pending_pixels = q[5];
-  out->slab_tasks = q[6];
-  out->slab_hits = q[7];
+  out->slab_tasks = q[6] - q[12];  // without the marches the walk left open
+  out->slab_hits = q[7] - q[13];
   out->rewalk_pixels = q[9];
   out->full_trace_pixels = q[10];
   return VXE_OK;
@@ -1899,6 +1907,9 @@ constexpr size_t kStageHdr = 0, kStageReqs = 64,
 // Stored probes and slab tasks per viewport ray of a batch; rays past the
 // budget walk again with inline probes.
 constexpr uint32_t kBatchProbesPerRay = 4, kBatchSlabsPerRay = 2;
+// Slab bins of a batch (SlabSink::bits): its viewports stand all over the world.
+constexpr uint32_t kBatchSlabBits = 6;
+constexpr size_t kBatchCountBytes = 64 + (size_t)(4096u << (kBatchSlabBits + 1u)) * 4;
 
 vxe_status lane_resources(vxe_ctx* c, BatchLane& L, uint32_t tiles, uint32_t vp_rays, uint32_t q_rays) {
   vxe_status st;
@@ -1931,6 +1942,7 @@ vxe_status lane_resources(vxe_ctx* c, BatchLane& L, uint32_t tiles, uint32_t vp_
     if ((st = alloc_on(c, L.px_probe, cap * 8, L.stream)) != VXE_OK) return st;
     if ((st = alloc_on(c, L.px_task, cap * 4, L.stream)) != VXE_OK) return st;
     if ((st = alloc_on(c, L.px_hit, cap * 64, L.stream)) != VXE_OK) return st;
+    if ((st = alloc_on(c, L.px_gov, cap * 16, L.stream)) != VXE_OK) return st;
     if ((st = alloc_on(c, L.q_pending, cap * 4, L.stream)) != VXE_OK) return st;
     if ((st = alloc_on(c, L.q_refine, cap * 4, L.stream)) != VXE_OK) return st;
     if ((st = alloc_on(c, L.q_far, cap * 4, L.stream)) != VXE_OK) return st;
@@ -1938,7 +1950,7 @@ vxe_status lane_resources(vxe_ctx* c, BatchLane& L, uint32_t tiles, uint32_t vp_
     if ((st = alloc_on(c, L.slab_tasks, cap * kBatchSlabsPerRay * 16, L.stream)) != VXE_OK) return st;
     if ((st = alloc_on(c, L.slab_res, cap * kBatchSlabsPerRay * 16, L.stream)) != VXE_OK) return st;
     if ((st = alloc_on(c, L.slab_hits, cap * kBatchSlabsPerRay * 4, L.stream)) != VXE_OK) return st;
-    if (!L.dcount.p && (st = alloc_on(c, L.dcount, 32, L.stream)) != VXE_OK) return st;
+    if (!L.dcount.p && (st = alloc_on(c, L.dcount, kBatchCountBytes, L.stream)) != VXE_OK) return st;
     L.ray_cap = (uint32_t)cap;
     if (L.graph) {  // the captured launches hold the old pointers
       cudaGraphExecDestroy(L.graph);
@@ -2010,6 +2022,8 @@ BatchArgs batch_args(const vxe_ctx* c, const BatchLane& L) {
   B.px_mask = (uint2*)L.px_mask.p;
   B.px_probe = (uint2*)L.px_probe.p;
   B.px_hit = (uint4*)L.px_hit.p;
+  B.px_gov = (uint4*)L.px_gov.p;
+  B.slab_bits = kBatchSlabBits;
   B.q_pending = (uint32_t*)L.q_pending.p;
   B.q_refine = (uint32_t*)L.q_refine.p;
   B.q_far = (uint32_t*)L.q_far.p;
@@ -2029,7 +2043,7 @@ vxe_status launch_persistent(vxe_ctx* c, BatchLane& L, const BatchArgs& B, bool 
                      L.stream));
   CK(cudaMemsetAsync(L.head.p, 0, 16, L.stream));
   if (B.defer) {
-    CK(cudaMemsetAsync(L.dcount.p, 0, 32, L.stream));
+    CK(cudaMemsetAsync(L.dcount.p, 0, 64 + (size_t)slab_bins(B.slab_bits) * 4, L.stream));
     k_batch_defer_clear<<<c->shade_wave, BATCH_THREADS, 0, L.stream>>>(B);
   }
   if (sorted) {
@@ -2045,6 +2059,8 @@ vxe_status launch_persistent(vxe_ctx* c, BatchLane& L, const BatchArgs& B, bool 
     k_batch_trace<false><<<c->b_trace_grid, BATCH_THREADS, 0, L.stream>>>(B);
   if (B.defer) {
     k_batch_probe_dda<<<c->shade_wave, BATCH_THREADS, 0, L.stream>>>(B);
+    k_batch_slab_bases<<<c->shade_wave, BATCH_THREADS, 0, L.stream>>>(B);
+    k_batch_slab_order<<<c->shade_wave, BATCH_THREADS, 0, L.stream>>>(B);
     k_batch_slab_eval<<<c->shade_wave, BATCH_THREADS, 0, L.stream>>>(B);
     k_batch_slab_pick<<<c->shade_wave, BATCH_THREADS, 0, L.stream>>>(B);
     k_batch_resolve<<<c->shade_wave, BATCH_THREADS, 0, L.stream>>>(B);

@@ -93,10 +93,11 @@ struct BatchArgs {
   uint4* px_hit;                  // 4 x uint4 per ray: voxel answer of a ray that met probes or needs refining
   uint4* px_gov;                  // per pending ray: the blade march its walk left open (FrameArgs::px_gov)
   uint32_t* q_pending;
-  uint32_t* q_refine;             // rays whose answer is a grass voxel (grass-slab refinement)
+  uint32_t* q_refine;             // rays whose answer is a grass voxel (grass-slab refinement); those that march go
+                                  // on in q_pending
   uint32_t* q_far;                // rays without a voxel answer (heightfield)
   uint32_t* dcount;               // [0] probes, [1] pending rays, [2] slab tasks, [3] slab hits, [4] refine, [5] far,
-                                  // [6] bin positions given out; from [16] the slab bins
+                                  // [6] bin positions given out, [7] refinement marches; from [16] the slab bins
   // coherent queries: query rays binned by (origin chunk, direction octant)
   uint32_t* q_keys;               // bin of each query ray
   uint32_t* q_perm;               // query rays in bin order
@@ -170,20 +171,12 @@ __device__ __noinline__ VoxTraceResult viewport_trace(const Scene& s, const uint
 // Record of voxel hit `best` (grass voxels get main_primary's grass-slab
 // refinement first).
 __device__ __noinline__ HitRec viewport_voxel_rec(const Scene& s, uint32_t gx, uint32_t gy, HitGeom best) {
-  const float vs = vs_(s);
   const v3 ro = cam_pos(s);
   const v3 rd = ray_dir_from_pixel(s, V2((float)gx + 0.5f, (float)gy + 0.5f));
-  if (best.mat == MAT_GRASS) {
-    const i3 ov{to_i32(floorf(best.root_bmin.x / vs + 0.5f)), to_i32(floorf(best.root_bmin.y / vs + 0.5f)),
-                to_i32(floorf(best.root_bmin.z / vs + 0.5f))};
-    const v3 hp = ro + rd * best.t;
-    const GrassCell cell =
-        pick_grass_cell_in_chunk_with_bias(hp, rd, best.root_bmin, ov, vs, (int32_t)s.cam->chunk_size);
-    const GrassHit gh = try_grass_slab_hit(s, ro, rd, 0.0f, best.t, cell.bmin_m, cell.id_vox, vs,
-                                           s.cam->voxel_params[1], s.cam->voxel_params[2]);
-    if (gh.hit) { best.t = gh.t; best.n = gh.n; }
-  }
-  return make_rec(best, ro, rd, vs, true);
+  GrassCell cell;
+  v2 iv;
+  if (grass_refine_setup(s, ro, rd, best, &cell, &iv)) grass_refine_march(s, ro, rd, cell, iv, best);
+  return make_rec(best, ro, rd, vs_(s), true);
 }
 
 // Record of a ray without a voxel hit: the heightfield (main_primary's
@@ -425,7 +418,7 @@ __global__ void __launch_bounds__(BATCH_THREADS) k_batch_defer_clear(const __gri
 }
 
 __device__ __forceinline__ SlabSink slab_sink(const BatchArgs& B) {
-  return SlabSink{reinterpret_cast<uint4*>(B.slab_res), B.slab_hits, &B.dcount[2], B.slab_cap, B.dcount + 16, B.slab_bits};
+  return SlabSink{reinterpret_cast<uint4*>(B.slab_res), &B.dcount[2], B.slab_cap, B.dcount + 16, B.slab_bits};
 }
 
 __global__ void __launch_bounds__(BATCH_THREADS) k_batch_probe_dda(const __grid_constant__ BatchArgs B) {
@@ -616,11 +609,32 @@ __global__ void __launch_bounds__(BATCH_THREADS) k_batch_resolve(const __grid_co
   }
 }
 
-__global__ void __launch_bounds__(BATCH_THREADS) k_batch_refine(const __grid_constant__ BatchArgs B) {
+// Rays whose answer is a grass voxel: most refinement marches miss at once
+// and are written here; the rest march one lane each in k_batch_refine.
+__global__ void __launch_bounds__(BATCH_THREADS) k_batch_refine_list(const __grid_constant__ BatchArgs B) {
   const uint32_t n_reqs = B.hdr->n_reqs;
   const uint32_t n = B.dcount[4];
   for (uint32_t i = blockIdx.x * BATCH_THREADS + threadIdx.x; i < n; i += gridDim.x * BATCH_THREADS) {
     const uint32_t ray = B.q_refine[i];
+    const BatchRay br = batch_ray(B, n_reqs, ray);
+    const Scene s = batch_scene(B, &B.cams[br.q->cam]);
+    const HitGeom best = load_pixhit(s, B.px_hit + (size_t)ray * 4u);
+    const v3 ro = cam_pos(s);
+    const v3 rd = ray_dir_from_pixel(s, V2((float)br.gx + 0.5f, (float)br.gy + 0.5f));
+    GrassCell cell;
+    v2 iv;
+    if (grass_refine_setup(s, ro, rd, best, &cell, &iv))
+      enqueue_active(B.q_pending, &B.dcount[7], ray);  // (the resolve is done with the pending queue)
+    else
+      store_rec_at(br.q->out, (size_t)br.gy * br.q->w + br.gx, make_rec(best, ro, rd, vs_(s), true));
+  }
+}
+
+__global__ void __launch_bounds__(BATCH_THREADS, SLAB_MIN_BLOCKS) k_batch_refine(const __grid_constant__ BatchArgs B) {
+  const uint32_t n_reqs = B.hdr->n_reqs;
+  const uint32_t n = B.dcount[7];
+  for (uint32_t i = blockIdx.x * BATCH_THREADS + threadIdx.x; i < n; i += gridDim.x * BATCH_THREADS) {
+    const uint32_t ray = B.q_pending[i];
     const BatchRay br = batch_ray(B, n_reqs, ray);
     const Scene s = batch_scene(B, &B.cams[br.q->cam]);
     const HitGeom best = load_pixhit(s, B.px_hit + (size_t)ray * 4u);

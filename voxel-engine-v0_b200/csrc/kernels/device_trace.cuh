@@ -1385,9 +1385,10 @@ __device__ __forceinline__ v3 slab_task_corner(const uint4& a, const Meta& ch, v
 // in a 1080p frame), so a warp then marches one or two cells: its lanes read
 // the same box frames (one L1 wavefront for all of them), run the same lod
 // and end after similar step counts.  A counting sort over bins of (lod, slot
-// hash, column): the append counts the bins and keeps each task's rank in its
-// bin; k_slab_bases turns counts into positions, k_slab_order moves the
-// tasks.  Cells that share a bin, and the order inside one, only cost time.
+// hash, column): the append counts the bins (an atomic without a result: the
+// column DDA's lanes diverge, and waiting there for ranks took 0.16 ms of a
+// 1080p frame); k_slab_bases turns counts into positions, k_slab_order moves
+// the tasks.  Cells that share a bin, and the order inside one, only cost time.
 // Unsorted, the marches ran 8.8 of 32 lanes and half of L1's wavefronts.
 // With the normals taken for nearest hits only and the marches the walk left
 // open among the tasks: 1080p frame 4.34 -> 3.66 ms, the 64-request batch
@@ -1395,10 +1396,9 @@ __device__ __forceinline__ v3 slab_task_corner(const uint4& a, const Meta& ch, v
 // 0.52 -> 0.53 ms.
 struct SlabSink {
   uint4* raw;          // tasks as found
-  uint32_t* rank;      // per task: its rank in its bin
   uint32_t* count;     // tasks found (beyond `cap`: not stored)
   uint32_t cap;
-  uint32_t* bins;      // slab_bins(bits) counters, then positions
+  uint32_t* bins;      // slab_bins(bits) counters, then next free positions
   uint32_t bits;       // slot hash bits of the lod-0 bins (1..6); one less at the other lods
 };
 __host__ __device__ __forceinline__ uint32_t slab_bins(uint32_t bits) { return 4096u << (bits + 1u); }
@@ -1412,7 +1412,7 @@ __device__ __forceinline__ bool slab_push(const SlabSink& k, const uint4& task) 
   const uint32_t j = atomicAdd(k.count, 1u);
   if (j >= k.cap) return false;
   k.raw[j] = task;
-  k.rank[j] = atomicAdd(&k.bins[slab_bin(task, k.bits)], 1u);
+  atomicAdd(&k.bins[slab_bin(task, k.bits)], 1u);
   return true;
 }
 // One lane per bin: its count becomes its first position; a warp's 32 bins
@@ -1436,7 +1436,7 @@ __device__ __forceinline__ void slab_order(const SlabSink& k, uint4* out) {
   const uint32_t n = min(*k.count, k.cap);
   for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
     const uint4 a = k.raw[j];
-    out[k.bins[slab_bin(a, k.bits)] + k.rank[j]] = a;
+    out[atomicAdd(&k.bins[slab_bin(a, k.bits)], 1u)] = a;
   }
 }
 

@@ -671,8 +671,9 @@ vxe_status frame_enqueue(vxe_ctx* c, FrameState& F, const FrameArgs& A, bool tim
       k_shade_far<1><<<grid(npix), SHADE_THREADS, 0, side->s>>>(A);
     }
     k_shade_prep<<<grid(npix), SHADE_THREADS, 0, st>>>(A);
+    k_shade_refine<<<grid(npix), SHADE_THREADS, 0, st>>>(A);
     if (side) {
-      // Every depth is final here (voxel pixels' from k_shade_prep, far
+      // Every depth is final here (voxel pixels' from k_shade_prep and k_shade_refine, far
       // pixels' from k_shade_far), and godray reads nothing else the shading
       // writes: it runs beside the rest of the voxel shading.
       CK(cudaEventRecord(side->prep, st));
@@ -746,6 +747,7 @@ vxe_status views_enqueue(vxe_ctx* c, const vxe::dev::FrameArgsViews& V, uint32_t
   CK(cudaStreamWaitEvent(side->s, side->mid, 0));
   k_shade_far_views<1><<<grid(max_pix), SHADE_THREADS, 0, side->s>>>(V);
   k_shade_prep_views<<<grid(max_pix), SHADE_THREADS, 0, st>>>(V);
+  k_shade_refine_views<<<grid(max_pix), SHADE_THREADS, 0, st>>>(V);
   CK(cudaEventRecord(side->prep, st));
   CK(cudaStreamWaitEvent(side->s, side->prep, 0));
   k_godray_views<<<dim3((max_iw + POST_THREADS_X - 1) / POST_THREADS_X, (max_ih + POST_THREADS_Y - 1) / POST_THREADS_Y, n),
@@ -2064,6 +2066,7 @@ vxe_status launch_persistent(vxe_ctx* c, BatchLane& L, const BatchArgs& B, bool 
     k_batch_slab_eval<<<c->shade_wave, BATCH_THREADS, 0, L.stream>>>(B);
     k_batch_slab_pick<<<c->shade_wave, BATCH_THREADS, 0, L.stream>>>(B);
     k_batch_resolve<<<c->shade_wave, BATCH_THREADS, 0, L.stream>>>(B);
+    k_batch_refine_list<<<c->shade_wave, BATCH_THREADS, 0, L.stream>>>(B);
     k_batch_refine<<<c->shade_wave, BATCH_THREADS, 0, L.stream>>>(B);
     k_batch_far<<<c->shade_wave, BATCH_THREADS, 0, L.stream>>>(B);
   }

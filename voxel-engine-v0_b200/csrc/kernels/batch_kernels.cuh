@@ -136,6 +136,7 @@ __device__ __forceinline__ Scene batch_scene(const BatchArgs& B, const vxe_camer
   s.grass_frames = table ? B.grass_frames : nullptr;
   s.slot_lights = nullptr;
   s.slot_top = nullptr;
+  s.sun_map = nullptr;
   return s;
 }
 

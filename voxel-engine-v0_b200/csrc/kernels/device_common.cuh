@@ -148,6 +148,10 @@ struct Scene {
   // the slot's non-air leaves, 0 when the slot holds none; null when the pass
   // has none.
   const uint32_t* __restrict__ slot_top;
+  // Sun horizon of the grid's columns for this frame (SUN_CELLS^2 cells per
+  // chunk column, world height in voxels; see sun_clear); null when the pass
+  // has none.
+  const float* __restrict__ sun_map;
 };
 
 struct Node { uint32_t child_base, child_mask, material, key; };

@@ -94,6 +94,9 @@ struct FrameArgs {
   float4* grass_frames;   // per record: the frames
   const uint32_t* slot_lights;  // per slot: holds a LIGHT leaf
   const uint32_t* slot_top;     // per slot: top of its non-air leaves (voxels)
+  const uint8_t* slot_cells;    // per slot: the same per SUN_CELL_VOX^2 columns (SUN_CELLS^2 bytes, z major)
+  float* sun_map;               // the grid's sun horizon (Scene::sun_map), then its cell tops, then their
+                                // maxima per chunk column; null: none
   uint32_t grass_slot0;  // k_grass_cells: first slot of the launch
   uint32_t* grass_list;    // grass columns of the last full build (k_grass_cells appends; null: no list)
   uint32_t* grass_list_n;  // their count
@@ -158,6 +161,7 @@ __device__ __forceinline__ Scene make_scene(const FrameArgs& A, bool godray) {
   s.grass_frames = A.grass_rec ? A.grass_frames : nullptr;
   s.slot_lights = A.slot_lights;
   s.slot_top = A.slot_top;
+  s.sun_map = A.sun_map;
   return s;
 }
 
@@ -261,8 +265,12 @@ constexpr int SLOT_LIGHT_THREADS = 256;
 __global__ void __launch_bounds__(SLOT_LIGHT_THREADS) k_slot_lights(const uint4* metas, uint64_t metas_n,
                                                                      const uint4* nodes, uint64_t nodes_n,
                                                                      uint32_t slot0, uint32_t chunk_size,
-                                                                     uint32_t* out, uint32_t* top_out) {
+                                                                     uint32_t* out, uint32_t* top_out,
+                                                                     uint8_t* cells_out) {
+  static_assert(SUN_CELLS * SUN_CELLS == SLOT_LIGHT_THREADS, "one thread per cell");
   __shared__ uint32_t top_s;
+  __shared__ uint32_t cell_s[SUN_CELLS * SUN_CELLS];
+  cell_s[threadIdx.x] = 0u;
   const uint32_t slot = slot0 + blockIdx.x;
   if (slot >= metas_n) return;
   if (threadIdx.x == 0) top_s = 0u;
@@ -277,15 +285,102 @@ __global__ void __launch_bounds__(SLOT_LIGHT_THREADS) k_slot_lights(const uint4*
     any |= (n.x == LEAF && n.z == MAT_LIGHT) ? 1 : 0;
     if (n.x == LEAF && n.z != MAT_AIR) {
       const uint32_t lvl = (n.w >> 18) & 7u, y = (n.w >> 6) & 63u;
-      top = max(top, (y + 1u) * (chunk_size >> lvl));
+      const uint32_t sz = chunk_size >> lvl, ltop = (y + 1u) * sz;
+      top = max(top, ltop);
+      // the cells under the leaf (one, or (sz / SUN_CELL_VOX)^2 for a larger leaf)
+      const uint32_t x0 = (n.w & 63u) * sz, z0 = ((n.w >> 12) & 63u) * sz;
+      for (uint32_t z = z0 / SUN_CELL_VOX; z * SUN_CELL_VOX < z0 + sz && z < SUN_CELLS; ++z)
+        for (uint32_t x = x0 / SUN_CELL_VOX; x * SUN_CELL_VOX < x0 + sz && x < SUN_CELLS; ++x)
+          if (cell_s[z * SUN_CELLS + x] < ltop) atomicMax(&cell_s[z * SUN_CELLS + x], ltop);
     }
   }
   atomicMax(&top_s, top);
   any = __syncthreads_or(any);
+  cells_out[(size_t)slot * (SUN_CELLS * SUN_CELLS) + threadIdx.x] = (uint8_t)min(cell_s[threadIdx.x], 255u);
   if (threadIdx.x == 0) {
     out[slot] = any ? 1u : 0u;
     top_out[slot] = top_s;
   }
+}
+
+// ---------------------------------------------------------------------------
+// Sun horizon of the grid (see sun_clear), one block per chunk column, one
+// thread per cell, made anew for each frame (a few microseconds beside the
+// walk: 65536 cells for 16 x 16 chunk columns), so it always is the world the
+// frame reads.
+// ---------------------------------------------------------------------------
+constexpr int SUN_THREADS = (int)(SUN_CELLS * SUN_CELLS);
+
+// The cell tops: world height (voxels) of the highest non-air leaf over each
+// cell.  A slot whose meta does not stand in its grid cell bars the shortcut
+// for its column.
+__global__ void __launch_bounds__(SUN_THREADS) k_sun_tops(const __grid_constant__ FrameArgs A) {
+  __shared__ float red[SUN_THREADS / 32];
+  const Scene s = make_scene(A, false);
+  const uint32_t nx = A.cam.grid_dims[0], ny = A.cam.grid_dims[1], nz = A.cam.grid_dims[2];
+  const uint32_t ix = blockIdx.x, iz = blockIdx.y, t = threadIdx.x;
+  float top = -BIG;
+  for (uint32_t iy = 0; iy < ny; ++iy) {
+    const uint32_t slot = grid_at(s, (iz * ny + iy) * nx + ix);
+    if (slot == INVALID || slot >= A.cam.chunk_count) continue;
+    const Meta m = meta_at(s, slot);
+    if (m.ox != (A.cam.grid_origin_chunk[0] + (int32_t)ix) * 64 || m.oy != (A.cam.grid_origin_chunk[1] + (int32_t)iy) * 64 ||
+        m.oz != (A.cam.grid_origin_chunk[2] + (int32_t)iz) * 64 || slot >= A.metas_n) {
+      top = BIG;
+      continue;
+    }
+    const uint32_t h = A.slot_cells[(size_t)slot * SUN_THREADS + t];
+    if (h != 0u) top = fmax_(top, (float)(m.oy + (int32_t)h));
+  }
+  const uint32_t cells = nx * nz * SUN_THREADS;
+  A.sun_map[cells + (iz * SUN_CELLS + t / SUN_CELLS) * (nx * SUN_CELLS) + ix * SUN_CELLS + t % SUN_CELLS] = top;
+  for (int o = 16; o; o >>= 1) top = fmax_(top, __shfl_xor_sync(0xFFFFFFFFu, top, o));
+  if ((t & 31u) == 0u) red[t >> 5] = top;
+  __syncthreads();
+  if (t == 0u) {
+    for (int k = 1; k < SUN_THREADS / 32; ++k) top = fmax_(top, red[k]);
+    A.sun_map[2u * cells + iz * nx + ix] = top;
+  }
+}
+
+// The horizon of each cell: the greatest top on the way of the sun rays that
+// start in it, less what they have risen on reaching it.  Such rays move
+// equally in +x and +z, so k cells on they cross only the cells (k, k),
+// (k + 1, k) and (k, k + 1), having gone more than k - 1 (the first) or k
+// (the others) cells along each axis.
+__global__ void __launch_bounds__(SUN_THREADS) k_sun_horizon(const __grid_constant__ FrameArgs A) {
+  const uint32_t nx = A.cam.grid_dims[0], nz = A.cam.grid_dims[2];
+  const uint32_t w = nx * SUN_CELLS, hgt = nz * SUN_CELLS, cells = w * hgt;
+  const float* top = A.sun_map + cells;
+  const float* col_top = top + cells;
+  // no cell of this column's rays is higher than the chunk columns they cross
+  __shared__ float bound_s;
+  if (threadIdx.x == 0u) {
+    float b = -BIG;
+    for (uint32_t k = 0; blockIdx.x + k < nx && blockIdx.y + k < nz; ++k) {
+      const uint32_t x = blockIdx.x + k, z = blockIdx.y + k;
+      b = fmax_(b, col_top[z * nx + x]);
+      if (x + 1u < nx) b = fmax_(b, col_top[z * nx + x + 1u]);
+      if (z + 1u < nz) b = fmax_(b, col_top[(z + 1u) * nx + x]);
+    }
+    bound_s = b;
+  }
+  __syncthreads();
+  const float bound = bound_s;
+  const uint32_t x0 = blockIdx.x * SUN_CELLS + threadIdx.x % SUN_CELLS, z0 = blockIdx.y * SUN_CELLS + threadIdx.x / SUN_CELLS;
+  // height gained per cell, rounded down
+  const float rise = (float)SUN_CELL_VOX * (SUN_Y / SUN_X) * 0.9999f;
+  static_assert(SUN_X == SUN_Z && SUN_X > 0.0f && SUN_Y > 0.0f, "the sun's rays run along the diagonal and rise");
+  float h = -BIG;
+  for (uint32_t k = 0; x0 + k < w && z0 + k < hgt; ++k) {
+    const float near = k == 0u ? 0.0f : rise * (float)(k - 1u), far = rise * (float)k;
+    if (bound - near <= h) break;
+    const uint32_t i = (z0 + k) * w + x0 + k;
+    h = fmax_(h, __ldg(&top[i]) - near);
+    if (x0 + k + 1u < w) h = fmax_(h, __ldg(&top[i + 1u]) - far);
+    if (z0 + k + 1u < hgt) h = fmax_(h, __ldg(&top[i + w]) - far);
+  }
+  A.sun_map[z0 * w + x0] = h;
 }
 
 // ---------------------------------------------------------------------------
@@ -1431,6 +1526,11 @@ __global__ void __launch_bounds__(SHADE_THREADS, SHADE_MIN_BLOCKS) k_shade_far_v
 // Godray pass
 // ---------------------------------------------------------------------------
 constexpr int POST_THREADS_X = 32, POST_THREADS_Y = 4;
+// Blocks per SM the godray kernels are compiled for: with most marches gone
+// (sun_clear) 64 registers are enough, where the march at every fourth sample
+// wanted 128 (4 blocks): k_godray 192 -> 178 us, k_godray_far 167 -> 157 us
+// (960x540 integrals).
+constexpr int GODRAY_MIN_BLOCKS = 8;
 
 // The godray ray of pixel (gx, gy) with depth t_c (main_godray,
 // ray_main.wgsl:520-535): the jittered direction and march length.
@@ -1528,12 +1628,12 @@ __device__ __forceinline__ void k_godray_far_body(const FrameArgs& A) {
     A.god_pre[pix] = make_float4(cur.x, cur.y, cur.z, 1.0f);
   }
 }
-__global__ void __launch_bounds__(SHADE_THREADS) k_godray_far(const __grid_constant__ FrameArgs A) { k_godray_far_body(A); }
-__global__ void __launch_bounds__(SHADE_THREADS) k_godray_far_views(const __grid_constant__ FrameArgsViews V) {
+__global__ void __launch_bounds__(SHADE_THREADS, GODRAY_MIN_BLOCKS) k_godray_far(const __grid_constant__ FrameArgs A) { k_godray_far_body(A); }
+__global__ void __launch_bounds__(SHADE_THREADS, GODRAY_MIN_BLOCKS) k_godray_far_views(const __grid_constant__ FrameArgsViews V) {
   k_godray_far_body(V.v[blockIdx.z]);
 }
-__global__ void __launch_bounds__(POST_THREADS_X* POST_THREADS_Y) k_godray(const __grid_constant__ FrameArgs A) { k_godray_body(A); }
-__global__ void __launch_bounds__(POST_THREADS_X* POST_THREADS_Y) k_godray_views(const __grid_constant__ FrameArgsViews V) {
+__global__ void __launch_bounds__(POST_THREADS_X* POST_THREADS_Y, GODRAY_MIN_BLOCKS) k_godray(const __grid_constant__ FrameArgs A) { k_godray_body(A); }
+__global__ void __launch_bounds__(POST_THREADS_X* POST_THREADS_Y, GODRAY_MIN_BLOCKS) k_godray_views(const __grid_constant__ FrameArgsViews V) {
   k_godray_body(V.v[blockIdx.z]);
 }
 
@@ -1704,6 +1804,7 @@ __device__ __forceinline__ Scene make_query_scene(const QueryArgs& Q) {
   s.grass_frames = nullptr;
   s.slot_lights = nullptr;
   s.slot_top = nullptr;
+  s.sun_map = nullptr;
   s.grass_taper = nullptr;
   return s;
 }

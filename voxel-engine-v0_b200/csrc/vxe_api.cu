@@ -102,12 +102,14 @@ struct SideStream {
   cudaStream_t s = nullptr;
   cudaEvent_t fork = nullptr, mid = nullptr, prep = nullptr, join = nullptr;
   cudaEvent_t pre = nullptr, table = nullptr;  // frame start -> side, grass table ready -> compute
+  cudaEvent_t sun_fork = nullptr, sun = nullptr;  // frame start -> side, sun horizon ready -> compute
 };
 
 struct BatchLane {
   cudaStream_t stream = nullptr;
   SideStream side;
   DevBuf hdr, reqs, cams, tile_count, tile_slots, head;
+  DevBuf sun;  // sun horizon of the views' frames on this lane
   // deferred grass probes of viewport rays: per-ray arrays for ray_cap rays,
   // probe records and slab tasks in proportion, counters
   DevBuf probe_recs, slab_tasks, slab_res, slab_hits, px_first, px_task, px_mask, px_probe, px_hit, px_gov, q_pending,
@@ -145,6 +147,8 @@ struct vxe_ctx {
   DevBuf nodes, ropes, metas, macro, colinfo, grid, clip_tex, errword;
   DevBuf slot_lights;  // per slot: holds a LIGHT leaf (k_slot_lights)
   DevBuf slot_top;     // per slot: top of its non-air leaves, voxels (k_slot_lights)
+  DevBuf slot_cells;   // per slot: the same per SUN_CELL_VOX^2 columns
+  DevBuf sun;          // sun horizon of the context's frames (SideStream's owner: lanes have their own)
   DevBuf profile;      // profile_counts of the context's frames (5 words)
   // caps on the wavefront's stored grass probes and slab tasks (0: the buffers' sizes)
   uint32_t probe_limit = 0, slab_limit = 0;
@@ -409,6 +413,26 @@ void fill_scene_args(const vxe_ctx* c, FrameArgs& A) {
   A.godray_alias = (c->flags & VXE_FLAG_GODRAY_MACRO_ALIAS) ? 1u : 0u;
   A.slot_lights = (const uint32_t*)c->slot_lights.p;
   A.slot_top = (const uint32_t*)c->slot_top.p;
+  A.slot_cells = (const uint8_t*)c->slot_cells.p;
+}
+
+// Bytes of one sun horizon (FrameArgs::sun_map): a grid has at most
+// grid_capacity chunk columns.
+size_t sun_bytes(const vxe_ctx* c) {
+  return (size_t)c->cfg.grid_capacity * (2u * vxe::dev::SUN_CELLS * vxe::dev::SUN_CELLS + 1u) * 4u;
+}
+
+// The horizon of the frame `A` on stream `st`, into A.sun_map (null: none).
+void sun_enqueue(const FrameArgs& A, cudaStream_t st) {
+  const uint32_t nx = A.cam.grid_dims[0], nz = A.cam.grid_dims[2];
+  if (!A.sun_map) return;
+  vxe::dev::k_sun_tops<<<dim3(nx, nz), vxe::dev::SUN_THREADS, 0, st>>>(A);
+  vxe::dev::k_sun_horizon<<<dim3(nx, nz), vxe::dev::SUN_THREADS, 0, st>>>(A);
+}
+// A grid that a horizon can be made for (a launch has at most 65535 rows).
+bool sun_usable(const vxe_camera_gpu& cam) {
+  return cam.chunk_count != 0 && cam.grid_dims[0] != 0 && cam.grid_dims[1] != 0 && cam.grid_dims[2] != 0 &&
+         cam.grid_dims[2] <= 65535u;
 }
 
 // Recomputes the light flags of slots [first, first + n) on the upload
@@ -417,7 +441,7 @@ vxe_status slot_lights_refresh(vxe_ctx* c, uint32_t first, uint32_t n) {
   if (n == 0 || !c->slot_lights.p) return VXE_OK;
   vxe::dev::k_slot_lights<<<n, vxe::dev::SLOT_LIGHT_THREADS, 0, c->upload>>>(
       (const uint4*)c->metas.p, c->cfg.chunk_capacity, (const uint4*)c->nodes.p, c->cfg.node_capacity, first, 64u,
-      (uint32_t*)c->slot_lights.p, (uint32_t*)c->slot_top.p);
+      (uint32_t*)c->slot_lights.p, (uint32_t*)c->slot_top.p, (uint8_t*)c->slot_cells.p);
   CK(cudaGetLastError());
   return VXE_OK;
 }
@@ -606,7 +630,7 @@ void frame_fill(vxe_ctx* c, FrameState& F, const vxe_camera_gpu& cam, FrameArgs&
 vxe_status side_ready(vxe_ctx* c, SideStream& S) {
   if (S.s) return VXE_OK;
   CK(cudaStreamCreateWithFlags(&S.s, cudaStreamNonBlocking));
-  for (cudaEvent_t* e : {&S.fork, &S.mid, &S.prep, &S.join, &S.pre, &S.table})
+  for (cudaEvent_t* e : {&S.fork, &S.mid, &S.prep, &S.join, &S.pre, &S.table, &S.sun_fork, &S.sun})
     CK(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
   return VXE_OK;
 }
@@ -616,7 +640,7 @@ void side_release(SideStream& S) {
     cudaStreamSynchronize(S.s);
     cudaStreamDestroy(S.s);
   }
-  for (cudaEvent_t e : {S.fork, S.mid, S.prep, S.join, S.pre, S.table})
+  for (cudaEvent_t e : {S.fork, S.mid, S.prep, S.join, S.pre, S.table, S.sun_fork, S.sun})
     if (e) cudaEventDestroy(e);
   S = SideStream{};
 }
@@ -627,6 +651,17 @@ vxe_status frame_enqueue(vxe_ctx* c, FrameState& F, const FrameArgs& A, bool tim
   const uint32_t tiles = tiles_x * tiles_y;
   const uint32_t npix = F.iw * F.ih;
   using namespace vxe::dev;
+  const bool beside = side && !(c->flags & VXE_FLAG_PRIMARY_MEGAKERNEL);
+  if (beside) {  // the sun horizon beside the walk
+    const vxe_status sr = side_ready(c, *side);
+    if (sr != VXE_OK) return sr;
+    CK(cudaEventRecord(side->sun_fork, st));
+    CK(cudaStreamWaitEvent(side->s, side->sun_fork, 0));
+    sun_enqueue(A, side->s);
+    CK(cudaEventRecord(side->sun, side->s));
+  } else {
+    sun_enqueue(A, st);
+  }
   if (timed) CK(cudaEventRecord(F.ev[1], st));
   k_tiles<<<(tiles + TILE_THREADS - 1) / TILE_THREADS, TILE_THREADS, 0, st>>>(A);
   if (timed) CK(cudaEventRecord(F.ev[2], st));
@@ -641,8 +676,6 @@ vxe_status frame_enqueue(vxe_ctx* c, FrameState& F, const FrameArgs& A, bool tim
                                                                 (uint64_t)c->shade_wave));
     };
     CK(cudaMemsetAsync(A.q_count, 0, kQcountBytes, st));
-    vxe_status sr;
-    if (side && (sr = side_ready(c, *side)) != VXE_OK) return sr;
     CK(cudaMemsetAsync(A.px_first, 0xFF, (size_t)npix * 8u, st));
     CK(cudaMemsetAsync(A.px_mask, 0, (size_t)npix * 8u, st));
     if (A.god_pre) CK(cudaMemsetAsync(A.god_pre, 0, (size_t)npix * 16u, st));
@@ -684,6 +717,7 @@ vxe_status frame_enqueue(vxe_ctx* c, FrameState& F, const FrameArgs& A, bool tim
       if (timed) CK(cudaEventRecord(F.ev[5], side->s));
       CK(cudaEventRecord(side->join, side->s));
     }
+    if (side) CK(cudaStreamWaitEvent(st, side->sun, 0));
     k_shade_shadow<<<grid(npix), SHADE_THREADS, 0, st>>>(A);
     k_shade_lights<<<grid((uint64_t)npix * 8u), SHADE_THREADS, 0, st>>>(A);
     k_shade_vox<<<grid(npix), SHADE_THREADS, 0, st>>>(A);
@@ -729,6 +763,11 @@ vxe_status views_enqueue(vxe_ctx* c, const vxe::dev::FrameArgsViews& V, uint32_t
   }
   vxe_status sr = side_ready(c, *side);
   if (sr != VXE_OK) return sr;
+  // one world, one sun horizon for all the views, beside their walks
+  CK(cudaEventRecord(side->sun_fork, st));
+  CK(cudaStreamWaitEvent(side->s, side->sun_fork, 0));
+  sun_enqueue(V.v[0], side->s);
+  CK(cudaEventRecord(side->sun, side->s));
   k_tiles_views<<<dim3((tiles_x * tiles_y + TILE_THREADS - 1) / TILE_THREADS, 1, n), TILE_THREADS, 0, st>>>(V);
   k_primary_trace_views<<<dim3((tiles_x + 1) / 2, tiles_y, n), PRIMARY_THREADS, 0, st>>>(V);
   for (uint32_t i = 0; i < n; ++i)  // the walk's far pixels shade beside the probe passes
@@ -753,6 +792,7 @@ vxe_status views_enqueue(vxe_ctx* c, const vxe::dev::FrameArgsViews& V, uint32_t
   k_godray_views<<<dim3((max_iw + POST_THREADS_X - 1) / POST_THREADS_X, (max_ih + POST_THREADS_Y - 1) / POST_THREADS_Y, n),
                    dim3(POST_THREADS_X, POST_THREADS_Y), 0, side->s>>>(V);
   CK(cudaEventRecord(side->join, side->s));
+  CK(cudaStreamWaitEvent(st, side->sun, 0));
   k_shade_shadow_views<<<grid(max_pix), SHADE_THREADS, 0, st>>>(V);
   k_shade_lights_views<<<grid(max_pix * 8u), SHADE_THREADS, 0, st>>>(V);
   k_shade_vox_views<<<grid(max_pix), SHADE_THREADS, 0, st>>>(V);
@@ -775,6 +815,7 @@ vxe_status launch_frame(vxe_ctx* c, bool timed) {
   FrameArgs A;
   frame_fill(c, c->fr, c->cam, A);
   A.profile = (uint32_t*)c->profile.p;
+  if (sun_usable(c->cam)) A.sun_map = (float*)c->sun.p;
   if (timed) CK(cudaEventRecord(c->fr.ev[0], c->compute));
   // In the wavefront schedule the walk reads nothing of the grass cell table
   // (its blade marches are deferred), so the table's per-frame rebuild runs
@@ -823,11 +864,13 @@ vxe_status launch_frame_graph(vxe_ctx* c, FrameState& F, const vxe_camera_gpu& c
   FrameArgs A;
   frame_fill(c, F, cam, A);
   if (&F == &c->fr) A.profile = (uint32_t*)c->profile.p;
+  if (&F == &c->fr && sun_usable(cam)) A.sun_map = (float*)c->sun.p;
   bool use_grass = false;
   if ((rc = grass_table_acquire(c, st, reader, cam, &use_grass)) != VXE_OK) return rc;
   if (use_grass) grass_table_args(c, A);
   const uint64_t key[8] = {F.iw, F.ih, F.pw, F.ph,
-                           (uint64_t)(c->flags & VXE_FLAG_PRIMARY_MEGAKERNEL) | (use_grass ? 2u : 0u),
+                           (uint64_t)(c->flags & VXE_FLAG_PRIMARY_MEGAKERNEL) | (use_grass ? 2u : 0u) |
+                               (A.sun_map ? (uint64_t)cam.grid_dims[0] << 2 | (uint64_t)cam.grid_dims[2] << 34 : 0u),
                            (uint64_t)c->shade_wave, (uint64_t)(uintptr_t)A.q_count, (uint64_t)(uintptr_t)A.px_first};
   if (!F.fgraph_exec || std::memcmp(key, F.fgraph_key, sizeof key) != 0) {
     if (F.fgraph_exec) cudaGraphExecDestroy(F.fgraph_exec);
@@ -961,6 +1004,8 @@ vxe_status vxe_create(const vxe_config* cfg, vxe_ctx** out) {
   if ((st = alloc(c, c->errword, 4)) != VXE_OK) return bail(st);
   if ((st = alloc(c, c->slot_lights, cc * 4)) != VXE_OK) return bail(st);
   if ((st = alloc(c, c->slot_top, cc * 4)) != VXE_OK) return bail(st);
+  if ((st = alloc(c, c->slot_cells, cc * (vxe::dev::SUN_CELLS * vxe::dev::SUN_CELLS))) != VXE_OK) return bail(st);
+  if ((st = alloc(c, c->sun, sun_bytes(c))) != VXE_OK) return bail(st);
   if ((st = alloc(c, c->profile, 32)) != VXE_OK) return bail(st);
   if (fill_sync(c->profile.p, 0, 32) != cudaSuccess) return bail(VXE_ERR_DEVICE);
   if (!(cfg->flags & VXE_FLAG_NO_GRASS_TABLE)) {
@@ -1005,13 +1050,13 @@ void vxe_destroy(vxe_ctx* c) {
   if (c->fr.fgraph) cudaGraphDestroy(c->fr.fgraph);
   for (auto& L : c->lanes)  // lanes read the arenas: drain them before freeing
     if (L.stream) cudaStreamSynchronize(L.stream);
-  for (auto* b : {&c->nodes, &c->ropes, &c->metas, &c->macro, &c->colinfo, &c->grid, &c->clip_tex, &c->errword, &c->slot_lights, &c->slot_top, &c->profile, &c->build_scratch, &c->build_places, &c->move_buf,
+  for (auto* b : {&c->nodes, &c->ropes, &c->metas, &c->macro, &c->colinfo, &c->grid, &c->clip_tex, &c->errword, &c->slot_lights, &c->slot_top, &c->slot_cells, &c->sun, &c->profile, &c->build_scratch, &c->build_places, &c->move_buf,
                   &c->q_in, &c->q_out, &c->gt.rec, &c->gt.taper, &c->gt.state, &c->gt.frames,
                   &c->gt.list, &c->gt.list_n})
     release(*b);
   for (auto& L : c->lanes) {
     if (L.stream) cudaStreamSynchronize(L.stream);
-    for (auto* b : {&L.hdr, &L.reqs, &L.cams, &L.tile_count, &L.tile_slots, &L.head, &L.probe_recs, &L.slab_tasks,
+    for (auto* b : {&L.hdr, &L.reqs, &L.cams, &L.tile_count, &L.tile_slots, &L.head, &L.sun, &L.probe_recs, &L.slab_tasks,
                     &L.slab_res, &L.slab_hits, &L.px_first, &L.px_task, &L.px_mask, &L.px_probe, &L.px_hit, &L.px_gov,
                     &L.q_pending, &L.q_refine, &L.q_far, &L.dcount, &L.q_keys, &L.q_perm, &L.bin_count})
       release(*b, L.stream);
@@ -2373,6 +2418,10 @@ vxe_status vxe_view_render_async(vxe_ctx* c, vxe_view* v, uint32_t lane, const v
   // launches (a view's graph would be re-captured whenever it changes lanes).
   FrameArgs A;
   frame_fill(c, v->fr, vc, A, &L.scratch);
+  if (sun_usable(vc)) {
+    if (!L.sun.p && (st = alloc_on(c, L.sun, sun_bytes(c), L.stream)) != VXE_OK) return st;
+    A.sun_map = (float*)L.sun.p;
+  }
   bool use_grass = false;
   const int reader = 1 + (int)lane;
   if ((st = grass_table_acquire(c, L.stream, reader, vc, &use_grass)) != VXE_OK) return st;
@@ -2453,10 +2502,13 @@ vxe_status vxe_view_render_batch_async(vxe_ctx* c, vxe_view* const* views, const
   std::memset(V, 0, sizeof *V);
   uint32_t max_iw = 0, max_ih = 0, max_pw = 0, max_ph = 0;
   uint64_t max_pix = 0, rays = 0;
+  const bool sun = sun_usable(vc[0]);
+  if (sun && !L.sun.p && (st = alloc_on(c, L.sun, sun_bytes(c), L.stream)) != VXE_OK) return st;
   for (uint32_t i = 0; i < n; ++i) {
     FrameState& F = views[i]->fr;
     frame_fill(c, F, vc[i], V->v[i], &L.mscratch[i]);
     if (use_grass) grass_table_args(c, V->v[i]);
+    if (sun) V->v[i].sun_map = (float*)L.sun.p;
     max_iw = std::max(max_iw, F.iw);
     max_ih = std::max(max_ih, F.ih);
     max_pw = std::max(max_pw, F.pw);

@@ -1083,12 +1083,12 @@ struct LeafState {
   uint32_t anchor_idx;
   v3 anchor_bmin;
   float anchor_size;
+  uint32_t key;  // of the leaf's node, or of the implicit leaf's anchor (the descent has loaded it)
 };
 
-__device__ AnchorNode anchor_from_leaf(const Scene& s, const LeafState& l, uint32_t node_base) {  // chunk_trace.wgsl:193-203
-  if (l.has_node) return AnchorNode{true, l.idx_local, l.bmin, l.size, node_key(s, node_base, l.idx_local)};
-  if (l.has_anchor)
-    return AnchorNode{true, l.anchor_idx, l.anchor_bmin, l.anchor_size, node_key(s, node_base, l.anchor_idx)};
+__device__ __forceinline__ AnchorNode anchor_from_leaf(const LeafState& l) {  // chunk_trace.wgsl:193-203
+  if (l.has_node) return AnchorNode{true, l.idx_local, l.bmin, l.size, l.key};
+  if (l.has_anchor) return AnchorNode{true, l.anchor_idx, l.anchor_bmin, l.anchor_size, l.key};
   return AnchorNode{false, 0, V3s(0.0f), 0.0f, INVALID};
 }
 
@@ -1118,33 +1118,35 @@ __device__ ExitFaceRes exit_face_from_slab_safe(v3 rd, const CubeSlab& slab) {  
   return ExitFaceRes{rd.z > 0.0f ? 4u : 5u, 0};
 }
 
-__device__ __forceinline__ LeafState descend_leaf_sparse(const Scene& s, v3 p, uint32_t node_base, uint32_t start_idx, v3 start_bmin,
-                              float start_size) {  // chunk_trace.wgsl:296-358
+// `n`: the record of node `start_idx`.
+__device__ __forceinline__ LeafState descend_leaf_sparse(const Scene& s, v3 p, uint32_t node_base, Node n,
+                                                         uint32_t start_idx, v3 start_bmin,
+                                                         float start_size) {  // chunk_trace.wgsl:296-358
   uint32_t idx = start_idx;
   v3 bmin = start_bmin;
   float size = start_size;
   const uint32_t max_d = chunk_max_depth(s);
   for (uint32_t d = 0; d < 32; ++d) {
-    const Node n = node_at(s, node_base, idx);
-    if (n.child_base == LEAF) return LeafState{true, idx, bmin, size, n.material, false, 0, V3s(0.0f), 0.0f};
-    if (d >= max_d) return LeafState{true, idx, bmin, size, MAT_AIR, false, 0, V3s(0.0f), 0.0f};
+    if (n.child_base == LEAF) return LeafState{true, idx, bmin, size, n.material, false, 0, V3s(0.0f), 0.0f, n.key};
+    if (d >= max_d) return LeafState{true, idx, bmin, size, MAT_AIR, false, 0, V3s(0.0f), 0.0f, n.key};
     const float half = size * 0.5f;
     const v3 mid = bmin + V3s(half);
     const float e = 1e-6f * size;
     const uint32_t hx = p.x > mid.x + e ? 1u : 0u, hy = p.y > mid.y + e ? 1u : 0u, hz = p.z > mid.z + e ? 1u : 0u;
     const uint32_t ci = hx | (hy << 1) | (hz << 2);
     const v3 cb = bmin + V3(hx ? half : 0.0f, hy ? half : 0.0f, hz ? half : 0.0f);
-    if ((n.child_mask & (1u << ci)) == 0u) return LeafState{false, INVALID, cb, half, MAT_AIR, true, idx, bmin, size};
+    if ((n.child_mask & (1u << ci)) == 0u) return LeafState{false, INVALID, cb, half, MAT_AIR, true, idx, bmin, size, n.key};
     idx = n.child_base + child_rank(n.child_mask, ci);
     bmin = cb;
     size = half;
+    n = node_at(s, node_base, idx);
   }
-  return LeafState{false, INVALID, start_bmin, start_size, MAT_AIR, false, INVALID, V3s(0.0f), 0.0f};
+  return LeafState{false, INVALID, start_bmin, start_size, MAT_AIR, false, INVALID, V3s(0.0f), 0.0f, INVALID};
 }
 
 __device__ __noinline__ LeafState descend_leaf_sparse_ool(const Scene& s, v3 p, uint32_t node_base, uint32_t start_idx,
                                                          v3 start_bmin, float start_size) {
-  return descend_leaf_sparse(s, p, node_base, start_idx, start_bmin, start_size);
+  return descend_leaf_sparse(s, p, node_base, node_at(s, node_base, start_idx), start_idx, start_bmin, start_size);
 }
 
 struct MacroDDAState {
@@ -1646,8 +1648,11 @@ __device__ __forceinline__ ChunkTraceResult trace_chunk_rope_interval_nomacro(co
   LeafState leaf{};
   // A descent chosen at the end of an air step (rope neighbour or anchor) is
   // made at the top of the next iteration, at the same point, so that the walk
-  // has one descent site.
+  // has one descent site.  Its first node is loaded when it is chosen: a rope
+  // neighbour's key and record are one load, and the anchor update takes the
+  // keys from the descent, so a step's chain has two loads fewer.
   bool pend = false, pend_anchor = false;
+  Node pend_node{0u, 0u, 0u, 0u};
   uint32_t pend_idx = 0u;
   v3 pend_bmin = V3s(0.0f);
   float pend_size = 0.0f;
@@ -1680,9 +1685,9 @@ __device__ __forceinline__ ChunkTraceResult trace_chunk_rope_interval_nomacro(co
       } else {
         break;
       }
-      leaf = descend_leaf_sparse(s, pq, ch.node_base, si, sb, ss);
+      leaf = descend_leaf_sparse(s, pq, ch.node_base, pending ? pend_node : node_at(s, ch.node_base, si), si, sb, ss);
       if (upd) {
-        const AnchorNode na = anchor_from_leaf(s, leaf, ch.node_base);
+        const AnchorNode na = anchor_from_leaf(leaf);
         if (na.valid && (!an.valid || na.key != an.key)) an = na;
       }
       have_leaf = true;
@@ -1735,13 +1740,15 @@ __device__ __forceinline__ ChunkTraceResult trace_chunk_rope_interval_nomacro(co
           pend_idx = leaf.anchor_idx;
           pend_bmin = leaf.anchor_bmin;
           pend_size = leaf.anchor_size;
+          pend_node = node_at(s, ch.node_base, pend_idx);
           continue;
         }
       }
       // the rope of the leaf's node, or of the implicit leaf's anchor
       const uint32_t nidx = rope_face(s, ch.node_base + (leaf.has_node ? leaf.idx_local : leaf.anchor_idx), face);
       if (nidx == INVALID) { have_leaf = false; continue; }
-      const v4 c = node_cube_from_key(rb, rs, node_key(s, ch.node_base, nidx));
+      pend_node = node_at(s, ch.node_base, nidx);
+      const v4 c = node_cube_from_key(rb, rs, pend_node.key);
       pend = true;
       pend_anchor = true;
       pend_idx = nidx;
@@ -1795,7 +1802,7 @@ __device__ __forceinline__ ChunkTraceResult trace_chunk_rope_interval_nomacro(co
     // descent still updates the anchor the walk returns
     const v3 pq = (ro + rd * tcur) + ray_eps_vec(rd, 1e-4f * vs);
     const LeafState l2 = descend_leaf_sparse_ool(s, pq, ch.node_base, pend_idx, pend_bmin, pend_size);
-    const AnchorNode na = anchor_from_leaf(s, l2, ch.node_base);
+    const AnchorNode na = anchor_from_leaf(l2);
     if (na.valid && (!an.valid || na.key != an.key)) an = na;
   }
   return ChunkTraceResult{miss_hitgeom(), an.valid, an.key};

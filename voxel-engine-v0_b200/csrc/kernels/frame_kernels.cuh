@@ -701,10 +701,14 @@ __device__ __forceinline__ PrimaryHint primary_hint(const Scene& s, const FrameA
 }
 
 // History hint + voxel trace (ray_main.wgsl:274-325 and trace_primary_voxels :116-161).
+// Inlined into the walk kernel, where the scene's fields are operands in the
+// constant bank: out of line they are reloaded from the caller's stack on the
+// walk's chains (L1 wavefronts 13.5 -> 7.4 % of peak, walk 739 -> 694 us per
+// 1080p frame; with the descent's loads shared, see pend_node, 689 us).
 template <uint32_t PM>
-__device__ __noinline__ VoxTraceResult primary_trace(const Scene& s, const FrameArgs& A, const PrimaryCtx& c,
-                                                     const uint32_t* cslot, const Meta* cmeta, uint32_t tile_count,
-                                                     ProbeHook& ph) {
+__device__ __forceinline__ VoxTraceResult primary_trace_inl(const Scene& s, const FrameArgs& A, const PrimaryCtx& c,
+                                                            const uint32_t* cslot, const Meta* cmeta,
+                                                            uint32_t tile_count, ProbeHook& ph) {
   VoxTraceResult vt{false, miss_hitgeom(), 0.0f, false, INVALID, i3{0, 0, 0}};
   if (s.cam->chunk_count == 0u || tile_count == 0u) return vt;
   const PrimaryHint hh = primary_hint(s, A, c);
@@ -720,6 +724,13 @@ __device__ __noinline__ VoxTraceResult primary_trace(const Scene& s, const Frame
                              w ? hh.anchor_key : INVALID, tile_count, ph);
     if (!w || h.best.hit != 0u) return h;
   }
+}
+
+template <uint32_t PM>
+__device__ __noinline__ VoxTraceResult primary_trace(const Scene& s, const FrameArgs& A, const PrimaryCtx& c,
+                                                     const uint32_t* cslot, const Meta* cmeta, uint32_t tile_count,
+                                                     ProbeHook& ph) {
+  return primary_trace_inl<PM>(s, A, c, cslot, cmeta, tile_count, ph);
 }
 
 // PROFILE_VOXEL of trace_primary_voxels (ray_main.wgsl:130-148): the tile's
@@ -1045,7 +1056,7 @@ __device__ __forceinline__ void k_primary_trace_body(const FrameArgs& A) {
     const PrimaryCtx c = primary_ctx(s, gx, gy, A.iw);
     pix = (uint32_t)c.pix;
     ProbeHook ph = probe_hook_record(A, pix);
-    const VoxTraceResult vt = primary_trace<PROBE_RECORD>(s, A, c, cslot[t], cmeta[t], ccount[t], ph);
+    const VoxTraceResult vt = primary_trace_inl<PROBE_RECORD>(s, A, c, cslot[t], cmeta[t], ccount[t], ph);
     walk_finish(A, pix, vt, ph, ccount[t], &vox, &pend);
     full = ph.first_phase <= 1u && ph.phase == 1u;
   }

@@ -39,8 +39,8 @@ struct BatchReq {  // 80 B
 
 struct BatchHeader {
   uint32_t n_reqs, total_tiles, n_items, tile_w, tile_h, rpt, tile_reqs, vp_rays;
-  // coherent queries: items >= vp_items take query rays in sorted order
-  uint32_t vp_items, q_rays, nbins, sorted;
+  // coherent queries (k_batch_queries): rays in sorted order, q_unit per warp
+  uint32_t vp_items, q_rays, nbins, sorted, q_unit;
 };
 
 struct BatchArgs {
@@ -65,7 +65,7 @@ struct BatchArgs {
   const vxe_camera_gpu* cams;
   uint32_t* tile_count;
   uint32_t* tile_slots;
-  uint32_t* head;       // [0] item counter, [1] tile counter
+  uint32_t* head;       // [0] item counter, [1] tile counter, [2] query counter
   uint32_t req_first;   // plain mode: the one request a launch serves
   uint32_t plain;       // 1: item = blockIdx-derived, no queue
   // grass cell table, valid for cameras with this wind time / strength
@@ -324,22 +324,31 @@ __device__ __forceinline__ void batch_item(const BatchArgs& B, const BatchHeader
   }
 }
 
-// Query rays in bin order (coherent mode): item k takes sorted positions
-// [k * 128 * rpt, ...); each lane finds its ray's request by the query base.
-__device__ __forceinline__ void batch_sorted_queries(const BatchArgs& B, const BatchHeader& H, uint32_t k,
-                                                     uint32_t lane) {
-  const uint32_t per = 128u * H.rpt;
-  for (uint32_t j = lane; j < per; j += 32u) {
-    const uint32_t pos = k * per + j;
-    if (pos >= H.q_rays) break;
-    const uint32_t ray = B.q_perm[pos];
-    const uint32_t r = find_req(B.reqs, H.n_reqs, ray, [](const BatchReq& q) { return q.q_base; });
-    const BatchReq& q = B.reqs[r];
-    const uint32_t i = ray - q.q_base;
-    const Scene s = batch_scene(B, &B.cams[0]);
-    const v3 ro = V3(q.o[3 * (size_t)i], q.o[3 * (size_t)i + 1], q.o[3 * (size_t)i + 2]);
-    const v3 rd = V3(q.d[3 * (size_t)i], q.d[3 * (size_t)i + 1], q.d[3 * (size_t)i + 2]);
-    store_rec_at(q.out, i, trace_query_ray(s, ro, rd, q.tmax));
+// Query rays in bin order: a warp takes the next q_unit sorted positions at a
+// time; each lane finds its ray's request by the query base.  A kernel of its
+// own beside the viewports': it holds the query walk alone (128 registers
+// against 168), and taking 32 rays at a time instead of 128 keeps every warp
+// busy when the rays are few.
+__global__ void __launch_bounds__(BATCH_THREADS) k_batch_queries(const __grid_constant__ BatchArgs B) {
+  const BatchHeader& H = *B.hdr;
+  const uint32_t lane = threadIdx.x & 31u, unit = H.q_unit, q_rays = H.q_rays, n_reqs = H.n_reqs;
+  const Scene s = batch_scene(B, &B.cams[0]);
+  for (;;) {
+    uint32_t k = 0;
+    if (lane == 0) k = atomicAdd(&B.head[2], 1u);
+    k = __shfl_sync(0xFFFFFFFFu, k, 0);
+    if (k * unit >= q_rays) break;
+    const uint32_t pos = k * unit + lane;
+    if (lane < unit && pos < q_rays) {
+      const uint32_t ray = B.q_perm[pos];
+      const uint32_t r = find_req(B.reqs, n_reqs, ray, [](const BatchReq& q) { return q.q_base; });
+      const BatchReq& q = B.reqs[r];
+      const uint32_t i = ray - q.q_base;
+      const v3 ro = V3(q.o[3 * (size_t)i], q.o[3 * (size_t)i + 1], q.o[3 * (size_t)i + 2]);
+      const v3 rd = V3(q.d[3 * (size_t)i], q.d[3 * (size_t)i + 1], q.d[3 * (size_t)i + 2]);
+      store_rec_at(q.out, i, trace_query_ray(s, ro, rd, q.tmax));
+    }
+    __syncwarp();
   }
 }
 
@@ -378,11 +387,7 @@ __global__ void __launch_bounds__(BATCH_THREADS) k_batch_trace(const __grid_cons
     uint32_t item = 0;
     if (lane == 0) item = atomicAdd(&B.head[0], 1u);
     item = __shfl_sync(0xFFFFFFFFu, item, 0);
-    if (item >= H.n_items) break;
-    if (H.sorted && item >= H.vp_items) {
-      batch_sorted_queries(B, H, item - H.vp_items, lane);
-      continue;
-    }
+    if (item >= H.vp_items) break;  // the queries are k_batch_queries'
     const uint32_t r = find_req(B.reqs, H.n_reqs, item, [](const BatchReq& q) { return q.item_begin; });
     const BatchReq q = B.reqs[r];
     load_cam(q.cam);

@@ -1785,6 +1785,7 @@ struct QueryArgs {
   const float* origins;
   const float* dirs;
   uint32_t n;
+  uint32_t unit;  // rays per warp (query_unit)
   float tmax;
   uint4* out;  // 2 x uint4 per ray
 };
@@ -1847,11 +1848,22 @@ __device__ __forceinline__ HitRec trace_query_ray(const Scene& s, v3 ro, v3 rd, 
   return miss_rec();
 }
 
-constexpr int QUERY_THREADS = 128;
+constexpr int QUERY_THREADS = 32;
 
+// Rays per warp of `n` queries on a GPU that holds `warps` of them: a warp
+// walks its rays' diverging paths one after another (64 rays in 2 warps take
+// twice as long as one ray a warp), so with fewer than 32 rays for every
+// resident warp the rays are spread over all of them, and more than 32 are
+// never taken at once.
+__host__ __device__ __forceinline__ uint32_t query_unit(uint64_t n, uint32_t warps) {
+  const uint64_t u = (n + warps - 1u) / warps;
+  return u < 1u ? 1u : u > 32u ? 32u : (uint32_t)u;
+}
+
+// One warp per block, `unit` rays each.
 __global__ void __launch_bounds__(QUERY_THREADS) k_query(const __grid_constant__ QueryArgs Q) {
-  const uint32_t i = blockIdx.x * QUERY_THREADS + threadIdx.x;
-  if (i >= Q.n) return;
+  const uint32_t i = blockIdx.x * Q.unit + threadIdx.x;
+  if (threadIdx.x >= Q.unit || i >= Q.n) return;
   const Scene s = make_query_scene(Q);
   const v3 ro = V3(Q.origins[3 * i], Q.origins[3 * i + 1], Q.origins[3 * i + 2]);
   const v3 rd = V3(Q.dirs[3 * i], Q.dirs[3 * i + 1], Q.dirs[3 * i + 2]);

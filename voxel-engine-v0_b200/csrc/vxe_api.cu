@@ -177,7 +177,7 @@ struct vxe_ctx {
   // batches: independent lanes (stream, pinned staging, descriptors, tile
   // lists, queue heads, captured graph) so several batches can be in flight
   BatchLane lanes[VXE_BATCH_LANES];
-  int b_trace_grid = 0, b_tile_grid = 0;
+  int b_trace_grid = 0, b_tile_grid = 0, b_query_grid = 0;
   int shade_wave = 148 * 16;  // blocks of the grid-stride shading kernels
   bool upload_recorded = false;
   // Stream-ordered pool for lane and view buffers: growing or freeing them
@@ -1916,7 +1916,8 @@ vxe_status vxe_trace_rays_device(vxe_ctx* c, const float* d_o, const float* d_d,
   Q.tmax = tmax;
   Q.out = (uint4*)d_out;
   using namespace vxe::dev;
-  k_query<<<(n + QUERY_THREADS - 1) / QUERY_THREADS, QUERY_THREADS, 0, c->compute>>>(Q);
+  Q.unit = query_unit(n, (uint32_t)c->shade_wave);  // 16 warps of 128 registers per SM
+  k_query<<<(n + Q.unit - 1) / Q.unit, QUERY_THREADS, 0, c->compute>>>(Q);
   CK(cudaGetLastError());
   return VXE_OK;
 }
@@ -1978,6 +1979,9 @@ vxe_status lane_resources(vxe_ctx* c, BatchLane& L, uint32_t tiles, uint32_t vp_
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&tb0, vxe::dev::k_batch_trace<false>, vxe::dev::BATCH_THREADS, 0));
     tb = std::min(tb, tb0);  // the persistent grid fills every SM for either instantiation
     CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&lb, vxe::dev::k_batch_tiles, vxe::dev::TILE_THREADS, 0));
+    int qb = 0;
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&qb, vxe::dev::k_batch_queries, vxe::dev::BATCH_THREADS, 0));
+    c->b_query_grid = sms * std::max(qb, 1);
     c->b_trace_grid = sms * std::max(tb, 1);
     c->b_tile_grid = sms * std::max(lb, 1);
   }
@@ -2099,12 +2103,17 @@ vxe_status launch_persistent(vxe_ctx* c, BatchLane& L, const BatchArgs& B, bool 
     k_qsort_scan<<<1, QSCAN_THREADS, 0, L.stream>>>(B);
     k_qsort_scatter<<<c->shade_wave, BATCH_THREADS, 0, L.stream>>>(B);
   }
-  k_batch_tiles<<<c->b_tile_grid, TILE_THREADS, 0, L.stream>>>(B);
-  if (B.defer)
-    k_batch_trace<true><<<c->b_trace_grid, BATCH_THREADS, 0, L.stream>>>(B);
-  else
-    k_batch_trace<false><<<c->b_trace_grid, BATCH_THREADS, 0, L.stream>>>(B);
+  if (sorted && !B.defer) {
+    k_batch_queries<<<c->b_query_grid, BATCH_THREADS, 0, L.stream>>>(B);
+  } else if (sorted) {  // beside the viewports: each fills what the other's tail leaves idle
+    CK(cudaEventRecord(L.side.fork, L.stream));
+    CK(cudaStreamWaitEvent(L.side.s, L.side.fork, 0));
+    k_batch_queries<<<c->b_query_grid, BATCH_THREADS, 0, L.side.s>>>(B);
+    CK(cudaEventRecord(L.side.join, L.side.s));
+  }
   if (B.defer) {
+    k_batch_tiles<<<c->b_tile_grid, TILE_THREADS, 0, L.stream>>>(B);
+    k_batch_trace<true><<<c->b_trace_grid, BATCH_THREADS, 0, L.stream>>>(B);
     k_batch_probe_dda<<<c->shade_wave, BATCH_THREADS, 0, L.stream>>>(B);
     k_batch_slab_bases<<<c->shade_wave, BATCH_THREADS, 0, L.stream>>>(B);
     k_batch_slab_order<<<c->shade_wave, BATCH_THREADS, 0, L.stream>>>(B);
@@ -2114,6 +2123,7 @@ vxe_status launch_persistent(vxe_ctx* c, BatchLane& L, const BatchArgs& B, bool 
     k_batch_refine_list<<<c->shade_wave, BATCH_THREADS, 0, L.stream>>>(B);
     k_batch_refine<<<c->shade_wave, BATCH_THREADS, 0, L.stream>>>(B);
     k_batch_far<<<c->shade_wave, BATCH_THREADS, 0, L.stream>>>(B);
+    if (sorted) CK(cudaStreamWaitEvent(L.stream, L.side.join, 0));
   }
   CK(cudaGetLastError());
   return VXE_OK;
@@ -2195,7 +2205,8 @@ vxe_status vxe_submit_batch_async(vxe_ctx* c, uint32_t lane, const vxe_request* 
   if (st != VXE_OK) return st;
   if (c->upload_recorded) CK(cudaStreamWaitEvent(L.stream, c->upload_done, 0));
   const uint32_t nbins = std::max(c->cfg.grid_capacity, 1u) * 8u;
-  BatchHeader H{n, tiles, items, tw, th, rpt, n, (uint32_t)vp_rays, vp_items, (uint32_t)q_rays, nbins, sorted ? 1u : 0u};
+  BatchHeader H{n, tiles, items, tw, th, rpt, n, (uint32_t)vp_rays, vp_items, (uint32_t)q_rays, nbins, sorted ? 1u : 0u,
+                query_unit(q_rays, (uint32_t)c->b_query_grid * (BATCH_THREADS / 32))};
   std::memcpy((char*)L.stage + kStageHdr, &H, sizeof H);
   if (n) std::memcpy((char*)L.stage + kStageReqs, R.data(), n * sizeof(BatchReq));
   auto* cams = (vxe_camera_gpu*)((char*)L.stage + kStageCams);
@@ -2214,6 +2225,7 @@ vxe_status vxe_submit_batch_async(vxe_ctx* c, uint32_t lane, const vxe_request* 
   }
   BatchArgs B = batch_args(c, L);
   B.defer = defer ? 1u : 0u;
+  if (defer && sorted && (st = side_ready(c, L.side)) != VXE_OK) return st;  // created outside a capture
   CK(cudaEventRecord(L.ev[0], L.stream));
   // Grass cell table for the wind of the first viewport's camera (requests
   // with another wind time / strength derive their cells in the march).

@@ -20,9 +20,11 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <initializer_list>
 #include <memory>
 #include <new>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "kernels/batch_kernels.cuh"
@@ -40,6 +42,7 @@ struct DevBuf {
   void* p = nullptr;
   size_t bytes = 0;
   bool pooled = false;  // from the context's stream-ordered pool
+  bool part = false;    // a part of another buffer (alloc_group), which owns the memory
 };
 
 enum Img {
@@ -145,6 +148,7 @@ struct vxe_ctx {
   bool upload_pending = false;
   // arenas
   DevBuf nodes, ropes, metas, macro, colinfo, grid, clip_tex, errword;
+  DevBuf small;        // owns metas, macro, ... (alloc_group)
   DevBuf slot_lights;  // per slot: holds a LIGHT leaf (k_slot_lights)
   DevBuf slot_top;     // per slot: top of its non-air leaves, voxels (k_slot_lights)
   DevBuf slot_cells;   // per slot: the same per SUN_CELL_VOX^2 columns
@@ -252,9 +256,27 @@ vxe_status alloc(vxe_ctx* c, DevBuf& b, size_t bytes) {
   return VXE_OK;
 }
 
+// Several buffers of a context in one allocation (`whole` owns it), zeroed
+// together: a cudaMalloc and its fill cost milliseconds of vxe_create each.
+vxe_status alloc_group(vxe_ctx* c, DevBuf& whole, std::initializer_list<std::pair<DevBuf*, size_t>> parts) {
+  size_t total = 0;
+  for (auto& q : parts) total += (q.second + 255) & ~(size_t)255;
+  const vxe_status st = alloc(c, whole, total);
+  if (st != VXE_OK) return st;
+  size_t at = 0;
+  for (auto& q : parts) {
+    *q.first = DevBuf{};
+    q.first->part = true;
+    q.first->bytes = q.second;
+    q.first->p = q.second ? (char*)whole.p + at : nullptr;
+    at += (q.second + 255) & ~(size_t)255;
+  }
+  return VXE_OK;
+}
+
 // Releases a buffer; a pooled one after the work queued on `st` so far.
 void release(DevBuf& b, cudaStream_t st = nullptr) {
-  if (b.p) {
+  if (b.p && !b.part) {
     if (b.pooled)
       cudaFreeAsync(b.p, st ? st : cudaStreamLegacy);
     else
@@ -262,7 +284,7 @@ void release(DevBuf& b, cudaStream_t st = nullptr) {
   }
   b.p = nullptr;
   b.bytes = 0;
-  b.pooled = false;
+  b.pooled = b.part = false;
 }
 
 // Stream-ordered (re)allocation from the context's pool, zero-filled on `st`.
@@ -994,26 +1016,21 @@ vxe_status vxe_create(const vxe_config* cfg, vxe_ctx** out) {
   const uint64_t nc = cfg->node_capacity, cc = cfg->chunk_capacity;
   if ((st = alloc(c, c->nodes, nc * 16)) != VXE_OK) return bail(st);
   if ((st = alloc(c, c->ropes, nc * 32)) != VXE_OK) return bail(st);
-  if ((st = alloc(c, c->metas, cc * 48)) != VXE_OK) return bail(st);
-  if ((st = alloc(c, c->macro, cc * VXE_MACRO_WORDS_PER_CHUNK * 4)) != VXE_OK) return bail(st);
-  if ((st = alloc(c, c->colinfo, cc * VXE_COLINFO_WORDS_PER_CHUNK * 4)) != VXE_OK) return bail(st);
-  if ((st = alloc(c, c->grid, (uint64_t)cfg->grid_capacity * 4)) != VXE_OK) return bail(st);
-  if (fill_sync(c->grid.p, 0xFF, c->grid.bytes) != cudaSuccess) return bail(VXE_ERR_DEVICE);
+  const bool table = !(cfg->flags & VXE_FLAG_NO_GRASS_TABLE);
   const uint64_t clip_bytes = (uint64_t)cfg->clip_levels * cfg->clip_res * cfg->clip_res * 4;
-  if ((st = alloc(c, c->clip_tex, clip_bytes)) != VXE_OK) return bail(st);
-  if ((st = alloc(c, c->errword, 4)) != VXE_OK) return bail(st);
-  if ((st = alloc(c, c->slot_lights, cc * 4)) != VXE_OK) return bail(st);
-  if ((st = alloc(c, c->slot_top, cc * 4)) != VXE_OK) return bail(st);
-  if ((st = alloc(c, c->slot_cells, cc * (vxe::dev::SUN_CELLS * vxe::dev::SUN_CELLS))) != VXE_OK) return bail(st);
-  if ((st = alloc(c, c->sun, sun_bytes(c))) != VXE_OK) return bail(st);
-  if ((st = alloc(c, c->profile, 32)) != VXE_OK) return bail(st);
-  if (fill_sync(c->profile.p, 0, 32) != cudaSuccess) return bail(VXE_ERR_DEVICE);
-  if (!(cfg->flags & VXE_FLAG_NO_GRASS_TABLE)) {
+  if ((st = alloc_group(c, c->small,
+                        {{&c->metas, cc * 48}, {&c->macro, cc * VXE_MACRO_WORDS_PER_CHUNK * 4},
+                         {&c->colinfo, cc * VXE_COLINFO_WORDS_PER_CHUNK * 4}, {&c->grid, (uint64_t)cfg->grid_capacity * 4},
+                         {&c->clip_tex, clip_bytes}, {&c->errword, 4}, {&c->slot_lights, cc * 4}, {&c->slot_top, cc * 4},
+                         {&c->slot_cells, cc * (vxe::dev::SUN_CELLS * vxe::dev::SUN_CELLS)}, {&c->sun, sun_bytes(c)},
+                         {&c->profile, 32}, {&c->gt.taper, table ? vxe::dev::GRASS_TAPER_N * 4u : 0u},
+                         {&c->gt.list_n, table ? 4u : 0u}})) != VXE_OK)
+    return bail(st);
+  if (fill_sync(c->grid.p, 0xFF, c->grid.bytes) != cudaSuccess) return bail(VXE_ERR_DEVICE);
+  if (table) {
     if ((st = alloc(c, c->gt.rec, cc * 4096u * vxe::dev::GRASS_REC_F4 * 16u)) != VXE_OK) return bail(st);
-    if ((st = alloc(c, c->gt.taper, vxe::dev::GRASS_TAPER_N * 4u)) != VXE_OK) return bail(st);
     if ((st = alloc(c, c->gt.state, cc * 4096u * 4u)) != VXE_OK) return bail(st);
     if ((st = alloc(c, c->gt.list, cc * 4096u * 4u)) != VXE_OK) return bail(st);
-    if ((st = alloc(c, c->gt.list_n, 4)) != VXE_OK) return bail(st);
     if ((st = alloc(c, c->gt.frames, cc * 4096u * vxe::dev::GRASS_FRAME_F4 * 16u)) != VXE_OK) return bail(st);
   }
   if (cudaEventCreateWithFlags(&c->gt.built, cudaEventDisableTiming) != cudaSuccess) return bail(VXE_ERR_DEVICE);
@@ -1052,7 +1069,7 @@ void vxe_destroy(vxe_ctx* c) {
     if (L.stream) cudaStreamSynchronize(L.stream);
   for (auto* b : {&c->nodes, &c->ropes, &c->metas, &c->macro, &c->colinfo, &c->grid, &c->clip_tex, &c->errword, &c->slot_lights, &c->slot_top, &c->slot_cells, &c->sun, &c->profile, &c->build_scratch, &c->build_places, &c->move_buf,
                   &c->q_in, &c->q_out, &c->gt.rec, &c->gt.taper, &c->gt.state, &c->gt.frames,
-                  &c->gt.list, &c->gt.list_n})
+                  &c->gt.list, &c->gt.list_n, &c->small})
     release(*b);
   for (auto& L : c->lanes) {
     if (L.stream) cudaStreamSynchronize(L.stream);

@@ -104,8 +104,10 @@ struct FrameArgs {
   // added to when cam.profile_flags & 1 (null: not counted)
   uint32_t* profile;
   // Godray integrals of the walk's far pixels, made beside the probe passes
-  // (k_godray_far; w = 1 where made, cleared each frame); null: none.
+  // (k_godray_far; w = the frame's tag where made, so that nothing needs
+  // clearing between frames); null: none.
   float4* god_pre = nullptr;
+  uint32_t god_tag = 0;
 };
 
 // profile_inc / profile_add (ray_main.wgsl:64-74).  The flag is uniform over
@@ -1013,6 +1015,8 @@ __device__ __forceinline__ void walk_finish(const FrameArgs& A, uint32_t pix, co
   const uint32_t gs = *vox ? vt.gov_state : 0u;
   *pend = ph.seq != 0u || gs != 0u;
   if (*pend) {
+    A.px_first[pix] = ~0ull;  // no probe hit yet
+    A.px_mask[pix] = make_uint2(0u, 0u);
     A.px_gov[pix] = make_uint4(gs, __float_as_uint(vt.gov_t0), __float_as_uint(vt.gov_t1), vt.gov_slot);
     // more probes than the summary counts: every stored one is still used,
     // the pixel just walks again
@@ -1594,7 +1598,7 @@ __device__ __forceinline__ void k_godray_body(const FrameArgs& A) {
   const GodrayPixel g = godray_pixel(s, gx, gy, t_c);
   const float4 pre = A.god_pre ? A.god_pre[(size_t)gy * W + gx] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   // made beside the probe passes for a far pixel of the walk
-  const v3 cur = pre.w != 0.0f ? V3(pre.x, pre.y, pre.z) : godray_pixel_integral(s, g);
+  const v3 cur = A.god_pre && __float_as_uint(pre.w) == A.god_tag ? V3(pre.x, pre.y, pre.z) : godray_pixel_integral(s, g);
   const v3 p_ws = ro + g.rd * t_hist;
   const v2 uvp = prev_uv_from_world(s, p_ws);
   v3 hl = cur;
@@ -1636,7 +1640,7 @@ __device__ __forceinline__ void k_godray_far_body(const FrameArgs& A) {
   for (uint32_t i = blockIdx.x * SHADE_THREADS + threadIdx.x; i < n; i += gridDim.x * SHADE_THREADS) {
     const uint32_t pix = A.q_far[i];
     const v3 cur = godray_pixel_integral(s, godray_pixel(s, pix % A.iw, pix / A.iw, A.depth[pix]));
-    A.god_pre[pix] = make_float4(cur.x, cur.y, cur.z, 1.0f);
+    A.god_pre[pix] = make_float4(cur.x, cur.y, cur.z, __uint_as_float(A.god_tag));
   }
 }
 __global__ void __launch_bounds__(SHADE_THREADS, GODRAY_MIN_BLOCKS) k_godray_far(const __grid_constant__ FrameArgs A) { k_godray_far_body(A); }

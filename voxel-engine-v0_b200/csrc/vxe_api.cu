@@ -93,10 +93,6 @@ struct FrameState {
   // set by launch_frame while an asynchronous read of the output image is in
   // flight: the composite (its writer) waits for it, the earlier passes do not
   cudaEvent_t composite_wait = nullptr;
-  // set by launch_frame when the grass cell table is (re)built on the side
-  // stream beside the walk: the first pass that reads the table (the blade
-  // marches) waits for it, the walk and the probe DDAs do not
-  cudaEvent_t table_wait = nullptr;
 };
 
 // A second stream a frame forks to (far-pixel shading beside the probe
@@ -104,7 +100,7 @@ struct FrameState {
 struct SideStream {
   cudaStream_t s = nullptr;
   cudaEvent_t fork = nullptr, mid = nullptr, prep = nullptr, join = nullptr;
-  cudaEvent_t pre = nullptr, table = nullptr;  // frame start -> side, grass table ready -> compute
+  cudaEvent_t pre = nullptr, table = nullptr;  // walk next -> side, grass table ready -> compute
   cudaEvent_t sun_fork = nullptr, sun = nullptr;  // frame start -> side, sun horizon ready -> compute
 };
 
@@ -182,6 +178,7 @@ struct vxe_ctx {
   // lists, queue heads, captured graph) so several batches can be in flight
   BatchLane lanes[VXE_BATCH_LANES];
   int b_trace_grid = 0, b_tile_grid = 0, b_query_grid = 0;
+  uint32_t god_tag = 0;  // FrameArgs::god_tag of the last frame filled
   int shade_wave = 148 * 16;  // blocks of the grid-stride shading kernels
   bool upload_recorded = false;
   // Stream-ordered pool for lane and view buffers: growing or freeing them
@@ -503,14 +500,18 @@ vxe_status grass_table_fill(vxe_ctx* c, cudaStream_t st, const vxe_camera_gpu& c
   return VXE_OK;
 }
 
+// Whether a pass with camera `cam` may read the table (once acquired).
+bool grass_table_usable(const vxe_ctx* c, const vxe_camera_gpu& cam) {
+  return c->gt.rec.p && !(c->flags & VXE_FLAG_NO_GRASS_TABLE) && cam.chunk_count != 0 &&
+         cam.chunk_count <= c->cfg.chunk_capacity;
+}
+
 // Makes the table valid on stream `st` for `cam`; *use tells whether the
 // pass may read it.  `reader` is the stream's index (0 compute, 1+ lanes).
 vxe_status grass_table_acquire(vxe_ctx* c, cudaStream_t st, int reader, const vxe_camera_gpu& cam, bool* use) {
   *use = false;
   GrassTable& T = c->gt;
-  if (!T.rec.p || (c->flags & VXE_FLAG_NO_GRASS_TABLE) || cam.chunk_count == 0 ||
-      cam.chunk_count > c->cfg.chunk_capacity)
-    return VXE_OK;
+  if (!grass_table_usable(c, cam)) return VXE_OK;
   const uint32_t tb = fbits(cam.voxel_params[1]), sb = fbits(cam.voxel_params[2]), vb = fbits(cam.voxel_params[0]);
   const bool same = T.valid && T.time_bits == tb && T.strength_bits == sb && T.vs_bits == vb &&
                     T.chunk_count == cam.chunk_count;
@@ -645,6 +646,7 @@ void frame_fill(vxe_ctx* c, FrameState& F, const vxe_camera_gpu& cam, FrameArgs&
   A.px_gov = (c->flags & VXE_FLAG_PRIMARY_MEGAKERNEL) ? nullptr : (uint4*)S->img[IMG_PXGOV].p;
   A.q_pending = (uint32_t*)S->img[IMG_QPENDING].p;
   A.god_pre = (c->flags & VXE_FLAG_PRIMARY_MEGAKERNEL) ? nullptr : (float4*)S->img[IMG_GODPRE].p;
+  A.god_tag = ++c->god_tag ? c->god_tag : ++c->god_tag;  // never 0, what the buffers start with
 }
 
 // The frame's launches on the compute stream (captured as-is by the graph
@@ -667,8 +669,10 @@ void side_release(SideStream& S) {
   S = SideStream{};
 }
 
+// `table_side`: A reads the grass cell table, which is made current here, on
+// the side stream beside the walk.
 vxe_status frame_enqueue(vxe_ctx* c, FrameState& F, const FrameArgs& A, bool timed, cudaStream_t st,
-                         SideStream* side) {
+                         SideStream* side, bool table_side = false) {
   const uint32_t tiles_x = (F.iw + 7) / 8, tiles_y = (F.ih + 7) / 8;
   const uint32_t tiles = tiles_x * tiles_y;
   const uint32_t npix = F.iw * F.ih;
@@ -698,12 +702,17 @@ vxe_status frame_enqueue(vxe_ctx* c, FrameState& F, const FrameArgs& A, bool tim
                                                                 (uint64_t)c->shade_wave));
     };
     CK(cudaMemsetAsync(A.q_count, 0, kQcountBytes, st));
-    CK(cudaMemsetAsync(A.px_first, 0xFF, (size_t)npix * 8u, st));
-    CK(cudaMemsetAsync(A.px_mask, 0, (size_t)npix * 8u, st));
-    if (A.god_pre) CK(cudaMemsetAsync(A.god_pre, 0, (size_t)npix * 16u, st));
+    if (table_side) CK(cudaEventRecord(side->pre, st));
     if (timed) CK(cudaEventRecord(F.ev[7], st));
     k_primary_trace<<<dim3((tiles_x + 1) / 2, tiles_y), PRIMARY_THREADS, 0, st>>>(A);
     if (timed) CK(cudaEventRecord(F.ev[8], st));
+    if (table_side) {  // the blades march after the walk: the table's rebuild fills the walk's tail
+      CK(cudaStreamWaitEvent(side->s, side->pre, 0));
+      bool use = false;
+      const vxe_status ts = grass_table_acquire(c, side->s, 0, A.cam, &use);
+      if (ts != VXE_OK) return ts;
+      CK(cudaEventRecord(side->table, side->s));
+    }
     if (side) {  // the walk's far pixels shade beside the probe passes
       CK(cudaMemcpyAsync(A.q_count + 8, A.q_count + 1, 4, cudaMemcpyDeviceToDevice, st));
       CK(cudaEventRecord(side->fork, st));
@@ -715,7 +724,7 @@ vxe_status frame_enqueue(vxe_ctx* c, FrameState& F, const FrameArgs& A, bool tim
     k_probe_dda<<<grid((uint64_t)npix * kProbesPerPixel), SHADE_THREADS, 0, st>>>(A);
     k_slab_bases<<<grid(slab_bins(kFrameSlabBits)), SHADE_THREADS, 0, st>>>(A);
     k_slab_order<<<grid((uint64_t)npix * kSlabsPerPixel), SHADE_THREADS, 0, st>>>(A);
-    if (F.table_wait) CK(cudaStreamWaitEvent(st, F.table_wait, 0));
+    if (table_side) CK(cudaStreamWaitEvent(st, side->table, 0));
     k_slab_eval<<<grid((uint64_t)npix * kSlabsPerPixel), SHADE_THREADS, 0, st>>>(A);
     k_slab_pick<<<grid(npix), SHADE_THREADS, 0, st>>>(A);
     k_primary_resolve<<<grid(npix), SHADE_THREADS, 0, st>>>(A);
@@ -775,14 +784,7 @@ vxe_status views_enqueue(vxe_ctx* c, const vxe::dev::FrameArgsViews& V, uint32_t
                                                                     (uint64_t)per_view)),
                 1, n);
   };
-  for (uint32_t i = 0; i < n; ++i) {
-    const FrameArgs& A = V.v[i];
-    const size_t npix = (size_t)A.iw * A.ih;
-    CK(cudaMemsetAsync(A.q_count, 0, kQcountBytes, st));
-    CK(cudaMemsetAsync(A.px_first, 0xFF, npix * 8u, st));
-    CK(cudaMemsetAsync(A.px_mask, 0, npix * 8u, st));
-    if (A.god_pre) CK(cudaMemsetAsync(A.god_pre, 0, npix * 16u, st));
-  }
+  for (uint32_t i = 0; i < n; ++i) CK(cudaMemsetAsync(V.v[i].q_count, 0, kQcountBytes, st));
   vxe_status sr = side_ready(c, *side);
   if (sr != VXE_OK) return sr;
   // one world, one sun horizon for all the views, beside their walks
@@ -841,25 +843,15 @@ vxe_status launch_frame(vxe_ctx* c, bool timed) {
   if (timed) CK(cudaEventRecord(c->fr.ev[0], c->compute));
   // In the wavefront schedule the walk reads nothing of the grass cell table
   // (its blade marches are deferred), so the table's per-frame rebuild runs
-  // on the side stream beside the tile lists and the walk; the blade marches
-  // wait for it.
-  const bool table_beside = !(c->flags & VXE_FLAG_PRIMARY_MEGAKERNEL);
-  cudaStream_t gst = c->compute;
-  if (table_beside) {
-    if ((st = side_ready(c, c->side)) != VXE_OK) return st;
-    CK(cudaEventRecord(c->side.pre, c->compute));
-    CK(cudaStreamWaitEvent(c->side.s, c->side.pre, 0));
-    gst = c->side.s;
-  }
-  bool use_grass = false;
-  if ((st = grass_table_acquire(c, gst, 0, c->cam, &use_grass)) != VXE_OK) return st;
+  // on the side stream, queued behind the walk's blocks (ahead of them it held
+  // the walk back for its whole 0.14 ms); the blade marches wait for it.
+  bool use_grass = grass_table_usable(c, c->cam);
+  const bool table_side = use_grass && !(c->flags & VXE_FLAG_PRIMARY_MEGAKERNEL);
+  if (!table_side && (st = grass_table_acquire(c, c->compute, 0, c->cam, &use_grass)) != VXE_OK) return st;
   if (use_grass) grass_table_args(c, A);
-  if (table_beside) CK(cudaEventRecord(c->side.table, gst));
-  c->fr.table_wait = table_beside ? c->side.table : nullptr;
   c->fr.composite_wait = c->out_pending ? c->out_ev : nullptr;
-  st = frame_enqueue(c, c->fr, A, timed, c->compute, &c->side);
+  st = frame_enqueue(c, c->fr, A, timed, c->compute, &c->side, table_side);
   c->fr.composite_wait = nullptr;
-  c->fr.table_wait = nullptr;
   if (st != VXE_OK) return st;
   c->out_pending = false;
   if (use_grass && (st = grass_table_release(c, c->compute, 0)) != VXE_OK) return st;

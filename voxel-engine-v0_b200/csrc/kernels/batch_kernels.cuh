@@ -154,7 +154,7 @@ __device__ __forceinline__ uint32_t find_req(const BatchReq* reqs, uint32_t n, u
 
 // Voxel trace of one cold viewport pixel (no history hint); PM the probe mode.
 template <uint32_t PM>
-__device__ __noinline__ VoxTraceResult viewport_trace(const Scene& s, const uint32_t* tile_count,
+__device__ __forceinline__ VoxTraceResult viewport_trace(const Scene& s, const uint32_t* tile_count,
                                                       const uint32_t* tile_slots, uint32_t tiles_x, uint32_t gx,
                                                       uint32_t gy, ProbeHook& ph) {
   const v3 ro = cam_pos(s);
@@ -331,25 +331,21 @@ __device__ __forceinline__ void batch_item(const BatchArgs& B, const BatchHeader
 // busy when the rays are few.
 __global__ void __launch_bounds__(BATCH_THREADS) k_batch_queries(const __grid_constant__ BatchArgs B) {
   const BatchHeader& H = *B.hdr;
-  const uint32_t lane = threadIdx.x & 31u, unit = H.q_unit, q_rays = H.q_rays, n_reqs = H.n_reqs;
+  const uint32_t n_reqs = H.n_reqs;
   const Scene s = batch_scene(B, &B.cams[0]);
-  for (;;) {
-    uint32_t k = 0;
-    if (lane == 0) k = atomicAdd(&B.head[2], 1u);
-    k = __shfl_sync(0xFFFFFFFFu, k, 0);
-    if (k * unit >= q_rays) break;
-    const uint32_t pos = k * unit + lane;
-    if (lane < unit && pos < q_rays) {
-      const uint32_t ray = B.q_perm[pos];
-      const uint32_t r = find_req(B.reqs, n_reqs, ray, [](const BatchReq& q) { return q.q_base; });
-      const BatchReq& q = B.reqs[r];
-      const uint32_t i = ray - q.q_base;
-      const v3 ro = V3(q.o[3 * (size_t)i], q.o[3 * (size_t)i + 1], q.o[3 * (size_t)i + 2]);
-      const v3 rd = V3(q.d[3 * (size_t)i], q.d[3 * (size_t)i + 1], q.d[3 * (size_t)i + 2]);
-      store_rec_at(q.out, i, trace_query_ray(s, ro, rd, q.tmax));
-    }
-    __syncwarp();
-  }
+  uint4* out = nullptr;
+  trace_query_rays(
+      s, QueryShare{&B.head[2], H.q_rays, H.q_unit, 0u, 0u},
+      [&](uint32_t pos, v3* ro, v3* rd, float* tmax) {
+        const uint32_t ray = B.q_perm[pos];
+        const BatchReq& q = B.reqs[find_req(B.reqs, n_reqs, ray, [](const BatchReq& r) { return r.q_base; })];
+        const size_t i = ray - q.q_base;
+        *ro = V3(q.o[3 * i], q.o[3 * i + 1], q.o[3 * i + 2]);
+        *rd = V3(q.d[3 * i], q.d[3 * i + 1], q.d[3 * i + 2]);
+        *tmax = q.tmax;
+        out = q.out + 2u * i;
+      },
+      [&](uint32_t, const HitRec& h) { store_rec(out, h); });
 }
 
 // The persistent work-queue kernel (plain = 0) or one request per launch

@@ -506,27 +506,39 @@ __device__ __forceinline__ BatchSlab batch_slab(const BatchArgs& B, uint32_t n_r
 }
 
 __global__ void __launch_bounds__(BATCH_THREADS, SLAB_MIN_BLOCKS) k_batch_slab_eval(const __grid_constant__ BatchArgs B) {
+  __shared__ SlabWarp work[BATCH_THREADS / 32];
   const uint32_t n_reqs = B.hdr->n_reqs;
-  const uint32_t n = min(B.dcount[2], B.slab_cap);
-  for (uint32_t j = blockIdx.x * BATCH_THREADS + threadIdx.x; j < n; j += gridDim.x * BATCH_THREADS) {
-    const BatchSlab w = batch_slab(B, n_reqs, j);
-    float t;
-    if (!slab_march(w.s, w.ro, w.rd, w.a, w.slot, w.cb, w.id, &t)) {
-      if (w.gov) B.px_gov[w.ray].x = 4u;  // the voxel hit stands
-      continue;
-    }
-    B.slab_res[j].x = t;
-    if (!w.gov) {
-      if (__float_as_uint(t) & 0x80000000u) {
-        atomicMin(&B.px_probe[w.ray].y, 0u);
-        continue;
-      }
-      const ProbeRec r = B.probe_recs[w.a.x];
-      const uint32_t cand = probe_cand(r), phase = probe_phase(r);
-      atomicMin(&B.px_first[w.ray], slab_key(phase, t, cand, probe_seq(r), slab_task_step(w.a)));
-      atomicOr(phase ? &B.px_mask[w.ray].y : &B.px_mask[w.ray].x, 1u << (cand & 31u));
-    }
-    B.slab_hits[atomicAdd(&B.dcount[3], 1u)] = j;
+  const uint32_t n = min(B.dcount[2], B.slab_cap), warps = gridDim.x * (BATCH_THREADS / 32);
+  const uint32_t chunk = n >= warps * SLAB_CHUNK ? SLAB_CHUNK : 32u;
+  for (uint32_t i = blockIdx.x * (BATCH_THREADS / 32) + (threadIdx.x >> 5); i * chunk < n; i += warps) {
+    slab_march_chunk(
+        work[threadIdx.x >> 5], i * chunk, chunk, n,
+        [&](uint32_t j, SlabRay* r) {
+          const BatchSlab w = batch_slab(B, n_reqs, j);
+          *r = SlabRay{w.a, w.slot, w.ro, w.rd, w.id, w.cb};
+          return w.s;
+        },
+        [&](uint32_t j, bool hit, float t) {
+          const uint4 a = B.slab_tasks[j];
+          if ((a.y & SLAB_GOV) != 0u) {
+            if (!hit) {
+              B.px_gov[a.x].x = 4u;  // the voxel hit stands
+              return;
+            }
+          } else {
+            if (!hit) return;
+            const ProbeRec r = B.probe_recs[a.x];
+            if (__float_as_uint(t) & 0x80000000u) {
+              atomicMin(&B.px_probe[r.pixel].y, 0u);
+              return;
+            }
+            const uint32_t cand = probe_cand(r), phase = probe_phase(r);
+            atomicMin(&B.px_first[r.pixel], slab_key(phase, t, cand, probe_seq(r), slab_task_step(a)));
+            atomicOr(phase ? &B.px_mask[r.pixel].y : &B.px_mask[r.pixel].x, 1u << (cand & 31u));
+          }
+          B.slab_res[j].x = t;
+          B.slab_hits[atomicAdd(&B.dcount[3], 1u)] = j;
+        });
   }
 }
 

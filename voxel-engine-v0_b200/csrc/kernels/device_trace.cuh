@@ -522,31 +522,45 @@ struct GrassSegFrame {
   float half_w, half_h;
 };
 
-__device__ __forceinline__ GrassSegFrame grass_seg_frame(const GrassBladeGeom& B, float blade_len, float inv_segs,
-                                                         float taper, uint32_t sg) {
-  const float t01a = (float)sg * inv_segs;
-  const float t01b = ((float)sg + 1.0f) * inv_segs;
-  const float ya = t01a * blade_len, yb = t01b * blade_len;
-  const float seg_h = yb - ya;
-  const float bend_a = (blade_len * t01a) * (0.55f + 0.45f * t01a);
-  const float bend_b = (blade_len * t01b) * (0.55f + 0.45f * t01b);
-  const v2 bva = B.w_xz * t01a + B.lean_dir * B.lean_amt;
-  const v2 bvb = B.w_xz * t01b + B.lean_dir * B.lean_amt;
-  const v2 offa = bva * bend_a, offb = bvb * bend_b;
-  const v3 pa = B.root + V3(offa.x, ya, offa.y);
-  const v3 pb = B.root + V3(offb.x, yb, offb.y);
+// A segment's end on the blade, at segment boundary k (0: the root).
+struct GrassSegEnd {
+  v3 p;
+  float y;
+};
+__device__ __forceinline__ GrassSegEnd grass_seg_end(const GrassBladeGeom& B, float blade_len, float inv_segs, uint32_t k) {
+  const float t01 = (float)k * inv_segs;
+  const float y = t01 * blade_len;
+  const float bend = (blade_len * t01) * (0.55f + 0.45f * t01);
+  const v2 off = (B.w_xz * t01 + B.lean_dir * B.lean_amt) * bend;
+  return GrassSegEnd{B.root + V3(off.x, y, off.y), y};
+}
+__device__ __forceinline__ GrassSegFrame grass_seg_between(const GrassBladeGeom& B, const GrassSegEnd& a,
+                                                           const GrassSegEnd& b, float taper) {
   GrassSegFrame f;
-  f.T = normalize(pb - pa);
+  f.T = normalize(b.p - a.p);
   v3 S = B.side_hint - f.T * dot(B.side_hint, f.T);
   const float s2 = dot(S, S);
   if (s2 < 1e-6f) S = ortho_basis_x(f.T);
   else S = S * (1.0f / sqrtf(s2));
   f.S = S;
-  f.N = cross(f.T, S);
-  f.mid = 0.5f * (pa + pb);
+  f.N = cross(f.T, f.S);
+  f.mid = 0.5f * (a.p + b.p);
   f.half_w = B.r0 * taper * 0.7f;
-  f.half_h = 0.5f * seg_h;
+  f.half_h = 0.5f * (b.y - a.y);
   return f;
+}
+// Calls `box` with the frames of a blade's segments in order (a segment's
+// lower end is the upper end of the one before).
+template <class F>
+__device__ __forceinline__ void grass_blade_boxes(const GrassBladeGeom& B, float blade_len, float inv_segs,
+                                                  uint32_t segs, const float* taper, F&& box) {
+  GrassSegEnd a = grass_seg_end(B, blade_len, inv_segs, 0u);
+#pragma unroll 1
+  for (uint32_t sg = 0; sg < segs; ++sg) {
+    const GrassSegEnd b = grass_seg_end(B, blade_len, inv_segs, sg + 1u);
+    box(grass_seg_between(B, a, b, taper[sg]), sg);
+    a = b;
+  }
 }
 
 // The minimum over boxes of sdf_box(local) = outside + inside (grass.wgsl:
@@ -743,13 +757,12 @@ __device__ __noinline__ bool grass_frames_ready(const Scene& s, GrassCellGeom& G
   if (v != 0u || atomicCAS(st, 0u, 1u) != 0u) return false;
   float4* F = s.grass_frames + G.rec * GRASS_FRAME_F4;
   for (uint32_t i = 0; i < G.blade_count; ++i)
-    for (uint32_t sg = 0; sg < G.segs; ++sg) {
-      const GrassSegFrame f = grass_seg_frame(G.blade[i], G.blade_len, G.inv_segs, G.taper[sg], sg);
+    grass_blade_boxes(G.blade[i], G.blade_len, G.inv_segs, G.segs, G.taper, [&](const GrassSegFrame& f, uint32_t sg) {
       float4* o = F + 3u * (i * G.segs + sg);
       o[0] = make_float4(f.mid.x, f.mid.y, f.mid.z, f.half_w);
       o[1] = make_float4(f.S.x, f.S.y, f.S.z, f.half_h);
       o[2] = make_float4(f.T.x, f.T.y, f.T.z, 0.0f);
-    }
+    });
   st_release_gpu(st, 2u);
   G.frames = 1u;
   return true;
@@ -791,8 +804,8 @@ __device__ __noinline__ float grass_sdf_cached(const Scene& s, v3 p, v3 cb, v3 i
     for (uint32_t k = 0; k < GRASS_FRAME_SEGS; ++k) grass_seg_sdf(m, grass_frame_load(F, k), p);
   } else {
     for (uint32_t i = 0; i < G.blade_count; ++i)
-      for (uint32_t sg = 0; sg < G.segs; ++sg)
-        grass_seg_sdf(m, grass_seg_frame(G.blade[i], G.blade_len, G.inv_segs, G.taper[sg], sg), p);
+      grass_blade_boxes(G.blade[i], G.blade_len, G.inv_segs, G.segs, G.taper,
+                        [&](const GrassSegFrame& f, uint32_t) { grass_seg_sdf(m, f, p); });
   }
   return sdf_min_value(m);
 }
@@ -860,9 +873,8 @@ __device__ __noinline__ v3 grass_sdf_normal_lod(const Scene& s, v3 p, v3 cb, v3 
       for (uint32_t k = 0; k < GRASS_FRAME_SEGS; ++k) box(grass_frame_load(F, k));
     } else {
       for (uint32_t i = 0; i < G.blade_count; ++i)
-#pragma unroll 1
-        for (uint32_t sg = 0; sg < G.segs; ++sg)
-          box(grass_seg_frame(G.blade[i], G.blade_len, G.inv_segs, G.taper[sg], sg));
+        grass_blade_boxes(G.blade[i], G.blade_len, G.inv_segs, G.segs, G.taper,
+                          [&](const GrassSegFrame& f, uint32_t) { box(f); });
     }
   });
 }
@@ -905,9 +917,8 @@ __device__ __forceinline__ float grass_sun_occlusion(const Scene& s, v3 p0, v3 s
       for (uint32_t k = 0; k < GRASS_FRAME_SEGS; ++k) box(grass_frame_load(F, k));
     } else {
       for (uint32_t b = 0; b < G.blade_count; ++b)
-#pragma unroll 1
-        for (uint32_t sg = 0; sg < G.segs; ++sg)
-          box(grass_seg_frame(G.blade[b], G.blade_len, G.inv_segs, G.taper[sg], sg));
+        grass_blade_boxes(G.blade[b], G.blade_len, G.inv_segs, G.segs, G.taper,
+                          [&](const GrassSegFrame& f, uint32_t) { box(f); });
     }
   }
   float occ = 0.0f;
@@ -1466,35 +1477,111 @@ __device__ __forceinline__ const float4* grass_column_frames(const Scene& s, uin
   return s.grass_frames + e * GRASS_FRAME_F4;
 }
 
-// March of a slab task's interval over cell (cb, id): grass_layer_march,
-// without the cell's blade geometry where the table has its box frames.
-__device__ __forceinline__ bool slab_march(const Scene& s, v3 ro, v3 rd, const uint4& a, uint32_t slot, v3 cb, v3 id,
-                                           float* t_hit) {
-  const float vs = vs_(s);
-  const float t0 = __uint_as_float(a.z), t1 = __uint_as_float(a.w);
-  const uint32_t lod = grass_lod_from_t(t0);
-  const float4* F = lod == 0u ? grass_column_frames(s, slot, a.y & 4095u, cb, id) : nullptr;
-  if (F == nullptr) {
-    GrassCellGeom G;
-    G.built = false;
-    return grass_layer_march(s, ro, rd, t0, t1, cb, id, s.cam->voxel_params[1], s.cam->voxel_params[2], lod, G, t_hit);
-  }
-  float t = t0;
-  for (uint32_t i = 0; i < GRASS_TRACE_STEPS; ++i) {
-    if (t > t1) break;
-    const v3 p = ro + rd * t;
-    if (!grass_in_layer(p, cb, vs)) break;  // a distance of BIG ends the march
-    SdfMin m = sdf_min_init();
-#pragma unroll 6
-    for (uint32_t k = 0; k < GRASS_FRAME_SEGS; ++k) grass_seg_sdf(m, grass_frame_load(F, k), p);
-    const float d = sdf_min_value(m);
-    if (d < GRASS_HIT_EPS_VOX * vs) {
-      *t_hit = t;
-      return true;
+// The marches of a warp's next `chunk` (32 or 64) sorted tasks, [base, base +
+// chunk) of n.  Marches over finished box frames (lod 0, nearly all of them)
+// take turns: a turn is one evaluation for the next 32 marches still alive in
+// the chunk, and the survivors queue up again, so lanes whose march has ended
+// after one of up to seven evaluations do not wait for the longest (14.6 of
+// 32 lanes before).  The others march in place (grass_layer_march).
+//   ray(j, &w)       task j's ray and cell; returns its scene
+//   done(j, hit, t)  its result, for every task of the chunk
+struct SlabRay {
+  uint4 a;
+  uint32_t slot;
+  v3 ro, rd, id, cb;
+};
+constexpr uint32_t SLAB_CHUNK = 64;
+struct SlabWarp {  // shared memory, one per warp
+  float ro[3][SLAB_CHUNK], rd[3][SLAB_CHUNK], cb[3][SLAB_CHUNK], t[SLAB_CHUNK], t1[SLAB_CHUNK], vs[SLAB_CHUNK];
+  uint32_t rec[SLAB_CHUNK];    // table record
+  uint8_t steps[SLAB_CHUNK];   // evaluations made; SLAB_HIT / SLAB_MISS at the end
+  uint8_t alive[SLAB_CHUNK];   // queue of the marches that go on
+};
+constexpr uint8_t SLAB_HIT = 254, SLAB_MISS = 255;
+template <class Ray, class Done>
+__device__ __forceinline__ void slab_march_chunk(SlabWarp& W, uint32_t base, uint32_t chunk, uint32_t n, Ray&& ray,
+                                                 Done&& done) {
+  const uint32_t lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
+  const float4* frames = nullptr;
+  uint32_t tail = 0u;
+  for (uint32_t r = 0; r < chunk; r += 32u) {
+    const uint32_t k = r + lane, j = base + k;
+    bool go = false;
+    if (j < n) {
+      SlabRay w;
+      const Scene s = ray(j, &w);
+      const float vs = vs_(s);
+      const float t0 = __uint_as_float(w.a.z), t1 = __uint_as_float(w.a.w);
+      const uint32_t lod = grass_lod_from_t(t0);
+      frames = s.grass_frames;
+      const float4* F = lod == 0u ? grass_column_frames(s, w.slot, w.a.y & 4095u, w.cb, w.id) : nullptr;
+      if (F == nullptr) {
+        GrassCellGeom G;
+        G.built = false;
+        float t = 0.0f;
+        const bool hit = grass_layer_march(s, w.ro, w.rd, t0, t1, w.cb, w.id, s.cam->voxel_params[1],
+                                           s.cam->voxel_params[2], lod, G, &t);
+        W.t[k] = t;
+        W.steps[k] = hit ? SLAB_HIT : SLAB_MISS;
+      } else {
+        // a first sample outside the layer (a distance of BIG) ends the march
+        go = !(t0 > t1) && grass_in_layer(w.ro + w.rd * t0, w.cb, vs);
+        W.ro[0][k] = w.ro.x; W.ro[1][k] = w.ro.y; W.ro[2][k] = w.ro.z;
+        W.rd[0][k] = w.rd.x; W.rd[1][k] = w.rd.y; W.rd[2][k] = w.rd.z;
+        W.cb[0][k] = w.cb.x; W.cb[1][k] = w.cb.y; W.cb[2][k] = w.cb.z;
+        W.t[k] = t0;
+        W.t1[k] = t1;
+        W.vs[k] = vs;
+        W.rec[k] = w.slot * 4096u + (w.a.y & 4095u);
+        W.steps[k] = go ? 0 : SLAB_MISS;
+      }
     }
-    t += fmax_(d, GRASS_STEP_MIN_VOX * vs);
+    const uint32_t m = __ballot_sync(0xFFFFFFFFu, go);
+    if (go) W.alive[tail + __popc(m & below)] = (uint8_t)k;
+    tail += (uint32_t)__popc(m);
   }
-  return false;
+  // (the scenes of a launch share the table: any lane's frames are all lanes')
+  for (uint32_t o = 16u; o; o >>= 1) {
+    const unsigned long long f = __shfl_xor_sync(0xFFFFFFFFu, (unsigned long long)(uintptr_t)frames, o);
+    if (frames == nullptr) frames = (const float4*)(uintptr_t)f;
+  }
+  __syncwarp();
+  for (uint32_t head = 0u; head < tail;) {
+    const uint32_t take = min(tail - head, 32u);
+    bool go = false;
+    uint32_t k = 0u;
+    if (lane < take) {
+      k = W.alive[(head + lane) % SLAB_CHUNK];
+      const v3 ro = V3(W.ro[0][k], W.ro[1][k], W.ro[2][k]), rd = V3(W.rd[0][k], W.rd[1][k], W.rd[2][k]);
+      float t = W.t[k];
+      const v3 p = ro + rd * t;
+      const float4* F = frames + (uint64_t)W.rec[k] * GRASS_FRAME_F4;
+      SdfMin m = sdf_min_init();
+#pragma unroll 6
+      for (uint32_t q = 0; q < GRASS_FRAME_SEGS; ++q) grass_seg_sdf(m, grass_frame_load(F, q), p);
+      const float d = sdf_min_value(m), vs = W.vs[k];
+      if (d < GRASS_HIT_EPS_VOX * vs) {
+        W.steps[k] = SLAB_HIT;  // at W.t
+      } else {
+        t += fmax_(d, GRASS_STEP_MIN_VOX * vs);
+        const uint32_t steps = W.steps[k] + 1u;
+        go = steps < GRASS_TRACE_STEPS && !(t > W.t1[k]) &&
+             grass_in_layer(ro + rd * t, V3(W.cb[0][k], W.cb[1][k], W.cb[2][k]), vs);
+        W.t[k] = t;
+        W.steps[k] = go ? (uint8_t)steps : SLAB_MISS;
+      }
+    }
+    const uint32_t m = __ballot_sync(0xFFFFFFFFu, go);  // every lane has read its place in the queue
+    if (go) W.alive[(tail + __popc(m & below)) % SLAB_CHUNK] = (uint8_t)k;
+    head += take;
+    tail += (uint32_t)__popc(m);
+    __syncwarp();
+  }
+  for (uint32_t r = 0; r < chunk; r += 32u) {
+    const uint32_t k = r + lane, j = base + k;
+    if (j < n) done(j, W.steps[k] == SLAB_HIT, W.t[k]);
+  }
+  __syncwarp();  // the next chunk overwrites the state
 }
 
 // The normal of a slab task's hit at t (grass_sdf_normal_lod).

@@ -218,14 +218,15 @@ __device__ __forceinline__ void grass_column_build(const FrameArgs& A, const Sce
     const uint32_t segs = grass_lod_segs(0u);
     const float inv_segs = 1.0f / fmax_((float)segs, 1.0f);
     float4* F = A.grass_frames + g * GRASS_FRAME_F4;
+    float taper[6];
+    for (uint32_t sg = 0; sg < segs; ++sg) taper[sg] = grass_taper_value(inv_segs, sg);
     for (uint32_t i = 0; i < GRASS_BLADE_COUNT; ++i)
-      for (uint32_t sg = 0; sg < segs; ++sg) {
-        const GrassSegFrame f = grass_seg_frame(B[i], blade_len, inv_segs, grass_taper_value(inv_segs, sg), sg);
+      grass_blade_boxes(B[i], blade_len, inv_segs, segs, taper, [&](const GrassSegFrame& f, uint32_t sg) {
         float4* o = F + 3u * (i * segs + sg);
         o[0] = make_float4(f.mid.x, f.mid.y, f.mid.z, f.half_w);
         o[1] = make_float4(f.S.x, f.S.y, f.S.z, f.half_h);
         o[2] = make_float4(f.T.x, f.T.y, f.T.z, 0.0f);
-      }
+      });
     A.grass_state[g] = 2u;
   }
 }
@@ -1170,29 +1171,40 @@ __device__ __forceinline__ SlabWork slab_work(const Scene& s, const FrameArgs& A
 // the normals, of the nearest hits only (13 % of the marches hit, and their
 // normals inside this kernel cost every warp about two more marches).
 __device__ __forceinline__ void k_slab_eval_body(const FrameArgs& A) {
+  __shared__ SlabWarp work[SHADE_THREADS / 32];
   const Scene s = make_scene(A, false);
-  const uint32_t n = min(A.q_count[6], A.slab_cap);
-  for (uint32_t j = blockIdx.x * SHADE_THREADS + threadIdx.x; j < n; j += gridDim.x * SHADE_THREADS) {
-    const SlabWork w = slab_work(s, A, j);
-    float t;
-    if (!slab_march(s, w.c.ro, w.c.rd, w.a, w.slot, w.cb, w.id, &t)) {
-      if (w.gov) A.px_gov[w.pix].x = 4u;  // the voxel hit stands
-      continue;
-    }
-    A.slab_res[j].x = t;
-    if (!w.gov) {
-      if (__float_as_uint(t) & 0x80000000u) {  // not ordered by the key: walk again
-        atomicMin(&A.px_probe[w.pix].y, 0u);
-        continue;
-      }
-      const ProbeRec r = A.probe_recs[w.a.x];
-      const uint32_t cand = probe_cand(r), phase = probe_phase(r);
-      atomicMin(&A.px_first[w.pix], slab_key(phase, t, cand, probe_seq(r), slab_task_step(w.a)));
-      atomicOr(phase ? &A.px_mask[w.pix].y : &A.px_mask[w.pix].x, 1u << (cand & 31u));
-    } else {
-      atomicAdd(&A.q_count[13], 1u);
-    }
-    A.slab_hits[atomicAdd(&A.q_count[7], 1u)] = j;
+  const uint32_t n = min(A.q_count[6], A.slab_cap), warps = gridDim.x * (SHADE_THREADS / 32);
+  const uint32_t chunk = n >= warps * SLAB_CHUNK ? SLAB_CHUNK : 32u;  // few tasks: over all the warps
+  for (uint32_t i = blockIdx.x * (SHADE_THREADS / 32) + (threadIdx.x >> 5); i * chunk < n; i += warps) {
+    slab_march_chunk(
+        work[threadIdx.x >> 5], i * chunk, chunk, n,
+        [&](uint32_t j, SlabRay* r) -> const Scene& {
+          const SlabWork w = slab_work(s, A, j);
+          *r = SlabRay{w.a, w.slot, w.c.ro, w.c.rd, w.id, w.cb};
+          return s;
+        },
+        [&](uint32_t j, bool hit, float t) {
+          const uint4 a = A.slab_tasks[j];
+          if ((a.y & SLAB_GOV) != 0u) {
+            if (!hit) {
+              A.px_gov[a.x].x = 4u;  // the voxel hit stands
+              return;
+            }
+            atomicAdd(&A.q_count[13], 1u);
+          } else {
+            if (!hit) return;
+            const ProbeRec r = A.probe_recs[a.x];
+            if (__float_as_uint(t) & 0x80000000u) {  // not ordered by the key: walk again
+              atomicMin(&A.px_probe[r.pixel].y, 0u);
+              return;
+            }
+            const uint32_t cand = probe_cand(r), phase = probe_phase(r);
+            atomicMin(&A.px_first[r.pixel], slab_key(phase, t, cand, probe_seq(r), slab_task_step(a)));
+            atomicOr(phase ? &A.px_mask[r.pixel].y : &A.px_mask[r.pixel].x, 1u << (cand & 31u));
+          }
+          A.slab_res[j].x = t;
+          A.slab_hits[atomicAdd(&A.q_count[7], 1u)] = j;
+        });
   }
 }
 __global__ void __launch_bounds__(SHADE_THREADS, SLAB_MIN_BLOCKS) k_slab_eval(const __grid_constant__ FrameArgs A) { k_slab_eval_body(A); }

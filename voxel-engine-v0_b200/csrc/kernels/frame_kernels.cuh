@@ -19,6 +19,8 @@
 namespace vxe {
 namespace dev {
 
+constexpr uint32_t QCOUNT_WORDS = 32;  // counters ahead of the slab bins
+
 struct FrameArgs {
   vxe_camera_gpu cam;
   vxe_clipmap_gpu clip;
@@ -63,8 +65,9 @@ struct FrameArgs {
   uint32_t* q_far;    // pixel ids for heightfield / sky
   uint32_t* q_count;  // [0] voxel, [1] far, [2] fresh shadow, [3] light gather, [4] probes, [5] pending,
                       // [6] slab tasks, [7] slab hits, [8] far pixels queued by the walk, [11] bin positions
-                      // given out, [12] / [13] the gov tasks / hits among [6] / [7], [14] refinement marches; then
-                      // the slab bins
+                      // given out, [12] / [13] the gov tasks / hits among [6] / [7], [14] refinement marches,
+                      // [15] pixels to walk again, [16] / [17] of them: voxel / far answers; from
+                      // QCOUNT_WORDS on the slab bins
   uint32_t* q_shadow;  // voxel pixels that trace a fresh sun shadow this frame
   uint32_t* q_light;   // voxel pixels that gather local lights
   float* px_shadow;    // fresh sun transmittance per pixel (q_shadow pixels)
@@ -86,6 +89,8 @@ struct FrameArgs {
                                   // interval, chunk slot); 3 / 4 once k_slab_pick / k_slab_eval ran it (hit / miss)
   uint32_t* q_pending;            // pixels whose walk met probes, q_count[5] of them; after the resolve, the
                                   // refinement marches (q_count[14])
+  uint32_t* q_walk;               // pixels the resolve could not decide, q_count[15] of them; once walked again,
+                                  // with WALKED_VOXEL where the answer is a voxel
   // per-frame grass cell table: written by k_grass_cells, read by the rest
   float4* grass_rec;
   uint64_t grass_rec_n;  // records (slots * 4096)
@@ -384,6 +389,16 @@ __global__ void __launch_bounds__(SUN_THREADS) k_sun_horizon(const __grid_consta
     if (z0 + k + 1u < hgt) h = fmax_(h, __ldg(&top[i + w]) - far);
   }
   A.sun_map[z0 * w + x0] = h;
+}
+
+// Rays per warp of `n` queries on a GPU that holds `warps` of them: a warp
+// walks its rays' diverging paths one after another (64 rays in 2 warps take
+// twice as long as one ray a warp), so with fewer than 32 rays for every
+// resident warp the rays are spread over all of them, and more than 32 are
+// never taken at once.
+__host__ __device__ __forceinline__ uint32_t query_unit(uint64_t n, uint32_t warps) {
+  const uint64_t u = (n + warps - 1u) / warps;
+  return u < 1u ? 1u : u > 32u ? 32u : (uint32_t)u;
 }
 
 // ---------------------------------------------------------------------------
@@ -1080,7 +1095,7 @@ __global__ void __launch_bounds__(PRIMARY_THREADS) k_primary_trace_views(const _
 // arguments, storing one task per grass slab it would march.  A probe whose
 // tasks do not all fit sends its pixel to the inline walk (stored count 0).
 __device__ __forceinline__ SlabSink slab_sink(const FrameArgs& A) {
-  return SlabSink{reinterpret_cast<uint4*>(A.slab_res), &A.q_count[6], A.slab_cap, A.q_count + 16, A.slab_bits};
+  return SlabSink{reinterpret_cast<uint4*>(A.slab_res), &A.q_count[6], A.slab_cap, A.q_count + QCOUNT_WORDS, A.slab_bits};
 }
 __device__ __forceinline__ void k_probe_dda_body(const FrameArgs& A) {
   const Scene s = make_scene(A, false);
@@ -1260,91 +1275,110 @@ __global__ void __launch_bounds__(SHADE_THREADS) k_slab_pick_views(const __grid_
   k_slab_pick_body(V.v[blockIdx.z]);
 }
 
-// Pixels that met probes: the nearer of the nearest probe hit and the voxel
+// A pixel that met probes: the nearer of the nearest probe hit and the voxel
 // answer (see the comment above ProbeRec), or, when that cannot be decided
-// from the parts, the reference walk with inline probes.
+// from the parts, the reference walk with inline probes.  Without WALK such a
+// pixel is left (*again).
+template <bool WALK>
+__device__ __forceinline__ bool resolve_pixel(const FrameArgs& A, const Scene& s, uint32_t pix, bool* again) {
+  const uint32_t tiles_x = (A.iw + 7u) / 8u;
+  const float vs = vs_(s);
+  bool vox = false;
+  *again = false;
+  const uint2 pp = A.px_probe[pix];
+  const uint32_t met = pp.x & 0xFFFFFFu;
+  uint32_t vcand = (pp.x >> 24) & 31u, vphase = (pp.x >> 29) & 1u;
+  uint32_t first_phase = (pp.x & 0x40000000u) != 0u ? 0u : 1u;
+  vox = (pp.x >> 31) != 0u;
+  if (A.px_gov != nullptr && A.px_gov[pix].x == 2u) {
+    // A deferred blade march left the voxel answer open: the walk again
+    // with its blade marches inline (probes only counted; their hits are
+    // the first walk's) gives the voxel answer, with the same probes
+    // before it.
+    if (!WALK) {
+      *again = true;
+      return false;
+    }
+    const uint32_t gx = pix % A.iw, gy = pix / A.iw;
+    const size_t tile = (size_t)(gy >> 3) * tiles_x + (gx >> 3);
+    const PrimaryCtx c = primary_ctx(s, gx, gy, A.iw);
+    ProbeHook ph = probe_hook_inline();
+    ph.mode = PROBE_RECORD;  // recs stay null: probes are counted, not stored
+    ph.pixel = pix;
+    const VoxTraceResult vt = primary_trace<PROBE_RECORD>(s, A, c, A.tile_slots + tile * TILE_CANDS, nullptr,
+                                                          A.tile_count[tile], ph);
+    vox = vt.in_grid && vt.best.hit != 0u;
+    if (vox) store_pixhit(A.pix_hit + (size_t)pix * 5u, vt.best, vt);
+    vcand = ph.best_cand & 31u;  // as probe_summary keeps it
+    vphase = ph.phase & 1u;
+    first_phase = ph.first_phase;
+  }
+  uint32_t answer_phase = vphase;  // phase of the answer (1 when there is none)
+  const unsigned long long first = A.px_first[pix];
+  bool walk = pp.y < met;  // some probes were not evaluated
+  if (!walk && first != ~0ull) {
+    const uint32_t j = A.px_task[pix];
+    const float4 res = A.slab_res[j];
+    const ProbeRec r = A.probe_recs[A.slab_tasks[j].x];
+    const uint32_t pcand = probe_cand(r), pphase = probe_phase(r);
+    bool probe_wins = true;
+    if (vox && pphase == vphase) {
+      const float vt = __uint_as_float(A.pix_hit[(size_t)pix * 5u].x);
+      probe_wins = res.x < vt || (res.x == vt && pcand <= vcand);
+    }
+    if (probe_wins) {
+      answer_phase = pphase;
+      const Meta ch = meta_at(s, r.slot);
+      const v3 rb = V3((float)ch.ox, (float)ch.oy, (float)ch.oz) * vs;
+      const float rs = (float)s.cam->chunk_size * vs;
+      const int32_t csz = (int32_t)s.cam->chunk_size;
+      const HitGeom g = make_hit(MAT_GRASS, res.x, V3(res.y, res.z, res.w), rb, rs, ch, r.node,
+                                 V3(r.leaf_bmin[0], r.leaf_bmin[1], r.leaf_bmin[2]), r.leaf_size);
+      const VoxTraceResult vr{true, g, 0.0f, probe_anchor_valid(r), r.anchor_key,
+                              i3{ch.ox / csz, ch.oy / csz, ch.oz / csz}};
+      store_pixhit(A.pix_hit + (size_t)pix * 5u, g, vr);
+      vox = true;
+    } else {
+      // the voxel answer's own chunk had a probe hit: undecided here
+      const uint2 pm = A.px_mask[pix];
+      walk = (((vphase ? pm.y : pm.x) >> vcand) & 1u) != 0u;
+    }
+  }
+  const uint32_t gx = pix % A.iw, gy = pix / A.iw;
+  const size_t tile = (size_t)(gy >> 3) * tiles_x + (gx >> 3);
+  if (walk && !WALK) {
+    *again = true;
+    return false;
+  }
+  if (walk) {
+    atomicAdd(&A.q_count[9], 1u);
+    const PrimaryCtx c = primary_ctx(s, gx, gy, A.iw);
+    ProbeHook ph = probe_hook_inline();
+    const VoxTraceResult vt = primary_trace<PROBE_INLINE>(s, A, c, A.tile_slots + tile * TILE_CANDS, nullptr,
+                                            A.tile_count[tile], ph);
+    vox = vt.in_grid && vt.best.hit != 0u;
+    if (vox) store_pixhit(A.pix_hit + (size_t)pix * 5u, vt.best, vt);
+    profile_voxel(A, ph.first_phase, ph.phase, A.tile_count[tile]);
+  } else {
+    profile_voxel(A, first_phase, vox ? answer_phase : 1u, A.tile_count[tile]);
+  }
+  return vox;
+}
+
 __device__ __forceinline__ void k_primary_resolve_body(const FrameArgs& A) {
   const Scene s = make_scene(A, false);
   const uint32_t n = A.q_count[5], end = warp_uniform_end(n);
-  const uint32_t tiles_x = (A.iw + 7u) / 8u;
-  const float vs = vs_(s);
   for (uint32_t i = blockIdx.x * SHADE_THREADS + threadIdx.x; i < end; i += gridDim.x * SHADE_THREADS) {
-    bool active = i < n, vox = false;
+    const bool active = i < n;
+    bool vox = false, again = false;
     uint32_t pix = 0u;
     if (active) {
       pix = A.q_pending[i];
-      const uint2 pp = A.px_probe[pix];
-      const uint32_t met = pp.x & 0xFFFFFFu;
-      uint32_t vcand = (pp.x >> 24) & 31u, vphase = (pp.x >> 29) & 1u;
-      uint32_t first_phase = (pp.x & 0x40000000u) != 0u ? 0u : 1u;
-      vox = (pp.x >> 31) != 0u;
-      if (A.px_gov != nullptr && A.px_gov[pix].x == 2u) {
-        // A deferred blade march left the voxel answer open: the walk again
-        // with its blade marches inline (probes only counted; their hits are
-        // the first walk's) gives the voxel answer, with the same probes
-        // before it.
-        const uint32_t gx = pix % A.iw, gy = pix / A.iw;
-        const size_t tile = (size_t)(gy >> 3) * tiles_x + (gx >> 3);
-        const PrimaryCtx c = primary_ctx(s, gx, gy, A.iw);
-        ProbeHook ph = probe_hook_inline();
-        ph.mode = PROBE_RECORD;  // recs stay null: probes are counted, not stored
-        ph.pixel = pix;
-        const VoxTraceResult vt = primary_trace<PROBE_RECORD>(s, A, c, A.tile_slots + tile * TILE_CANDS, nullptr,
-                                                              A.tile_count[tile], ph);
-        vox = vt.in_grid && vt.best.hit != 0u;
-        if (vox) store_pixhit(A.pix_hit + (size_t)pix * 5u, vt.best, vt);
-        vcand = ph.best_cand & 31u;  // as probe_summary keeps it
-        vphase = ph.phase & 1u;
-        first_phase = ph.first_phase;
-      }
-      uint32_t answer_phase = vphase;  // phase of the answer (1 when there is none)
-      const unsigned long long first = A.px_first[pix];
-      bool walk = pp.y < met;  // some probes were not evaluated
-      if (!walk && first != ~0ull) {
-        const uint32_t j = A.px_task[pix];
-        const float4 res = A.slab_res[j];
-        const ProbeRec r = A.probe_recs[A.slab_tasks[j].x];
-        const uint32_t pcand = probe_cand(r), pphase = probe_phase(r);
-        bool probe_wins = true;
-        if (vox && pphase == vphase) {
-          const float vt = __uint_as_float(A.pix_hit[(size_t)pix * 5u].x);
-          probe_wins = res.x < vt || (res.x == vt && pcand <= vcand);
-        }
-        if (probe_wins) {
-          answer_phase = pphase;
-          const Meta ch = meta_at(s, r.slot);
-          const v3 rb = V3((float)ch.ox, (float)ch.oy, (float)ch.oz) * vs;
-          const float rs = (float)s.cam->chunk_size * vs;
-          const int32_t csz = (int32_t)s.cam->chunk_size;
-          const HitGeom g = make_hit(MAT_GRASS, res.x, V3(res.y, res.z, res.w), rb, rs, ch, r.node,
-                                     V3(r.leaf_bmin[0], r.leaf_bmin[1], r.leaf_bmin[2]), r.leaf_size);
-          const VoxTraceResult vr{true, g, 0.0f, probe_anchor_valid(r), r.anchor_key,
-                                  i3{ch.ox / csz, ch.oy / csz, ch.oz / csz}};
-          store_pixhit(A.pix_hit + (size_t)pix * 5u, g, vr);
-          vox = true;
-        } else {
-          // the voxel answer's own chunk had a probe hit: undecided here
-          const uint2 pm = A.px_mask[pix];
-          walk = (((vphase ? pm.y : pm.x) >> vcand) & 1u) != 0u;
-        }
-      }
-      const uint32_t gx = pix % A.iw, gy = pix / A.iw;
-      const size_t tile = (size_t)(gy >> 3) * tiles_x + (gx >> 3);
-      if (walk) {
-        atomicAdd(&A.q_count[9], 1u);
-        const PrimaryCtx c = primary_ctx(s, gx, gy, A.iw);
-        ProbeHook ph = probe_hook_inline();
-        const VoxTraceResult vt = primary_trace<PROBE_INLINE>(s, A, c, A.tile_slots + tile * TILE_CANDS, nullptr,
-                                                A.tile_count[tile], ph);
-        vox = vt.in_grid && vt.best.hit != 0u;
-        if (vox) store_pixhit(A.pix_hit + (size_t)pix * 5u, vt.best, vt);
-        profile_voxel(A, ph.first_phase, ph.phase, A.tile_count[tile]);
-      } else {
-        profile_voxel(A, first_phase, vox ? answer_phase : 1u, A.tile_count[tile]);
-      }
+      vox = resolve_pixel<false>(A, s, pix, &again);
     }
     enqueue(A.q_vox, &A.q_count[0], active && vox, pix);
-    enqueue(A.q_far, &A.q_count[1], active && !vox, pix);
+    enqueue(A.q_far, &A.q_count[1], active && !vox && !again, pix);
+    enqueue(A.q_walk, &A.q_count[15], again, pix);
   }
 }
 __global__ void __launch_bounds__(SHADE_THREADS) k_primary_resolve(const __grid_constant__ FrameArgs A) { k_primary_resolve_body(A); }
@@ -1446,6 +1480,54 @@ __global__ void __launch_bounds__(SHADE_THREADS, SLAB_MIN_BLOCKS) k_shade_refine
   k_shade_refine_body(V.v[blockIdx.z]);
 }
 
+// The pixels the resolve could not decide (a few hundred of a frame), walked
+// again beside the refinement of the others: a walk is one lane's chain of
+// 0.1 ms and more, which the resolve used to end with.  Each is finished here
+// as far as its class goes -- far pixels shaded, voxel pixels refined and
+// classified -- so nothing that runs beside it reads its queues; k_shade_vox
+// shades the voxel answers from q_walk.  One pixel per warp while they fit.
+// Device frame 2.93 -> 2.87 ms at 1080p, 3.06 -> 2.98 ms with lights.  (The
+// same for batches, whose walks probe inline beside the refinement: 48.0 ->
+// 49.4 ms, so theirs stay in k_batch_resolve.)
+constexpr uint32_t WALKED_VOXEL = 0x80000000u;
+constexpr int WALK_THREADS = 32;
+__device__ __forceinline__ void k_primary_walk_body(const FrameArgs& A) {
+  const Scene s = make_scene(A, false);
+  const uint32_t n = A.q_count[15], unit = query_unit(n, gridDim.x), lane = threadIdx.x;
+  for (uint32_t i0 = blockIdx.x * unit; i0 < n; i0 += gridDim.x * unit) {
+    const uint32_t i = i0 + lane;
+    const bool active = lane < unit && i < n;
+    bool fresh = false, light = false;
+    uint32_t pix = 0u;
+    if (active) {
+      pix = A.q_walk[i];
+      bool again;
+      const bool vox = resolve_pixel<true>(A, s, pix, &again);
+      const PrimaryCtx c = primary_ctx(s, pix % A.iw, pix / A.iw, A.iw);
+      if (vox) {
+        uint4* src = A.pix_hit + (size_t)pix * 5u;
+        HitGeom g = load_pixhit(s, src);
+        if (grass_refine(s, c, g)) {
+          profile_add(A, PROFILE_GRASS, 1u);
+          src[0] = make_uint4(__float_as_uint(g.t), __float_as_uint(g.n.x), __float_as_uint(g.n.y),
+                              __float_as_uint(g.n.z));
+        }
+        shade_classify(A, s, c, g, &fresh, &light);
+        A.q_walk[i] = pix | WALKED_VOXEL;
+      } else {
+        shade_far_pixel(s, A, c);
+      }
+      atomicAdd(&A.q_count[vox ? 16 : 17], 1u);
+    }
+    enqueue(A.q_shadow, &A.q_count[2], fresh, pix);
+    enqueue(A.q_light, &A.q_count[3], light, pix);
+  }
+}
+__global__ void __launch_bounds__(WALK_THREADS) k_primary_walk(const __grid_constant__ FrameArgs A) { k_primary_walk_body(A); }
+__global__ void __launch_bounds__(WALK_THREADS) k_primary_walk_views(const __grid_constant__ FrameArgsViews V) {
+  k_primary_walk_body(V.v[blockIdx.z]);
+}
+
 __device__ __forceinline__ void k_shade_shadow_body(const FrameArgs& A) {
   const Scene s = make_scene(A, false);
   const uint32_t n = A.q_count[2];
@@ -1505,9 +1587,16 @@ __global__ void __launch_bounds__(SHADE_THREADS) k_shade_lights_views(const __gr
 
 __device__ __forceinline__ void k_shade_vox_body(const FrameArgs& A) {
   const Scene s = make_scene(A, false);
-  const uint32_t n = A.q_count[0];
+  const uint32_t nq = A.q_count[0], n = nq + A.q_count[15];
   for (uint32_t i = blockIdx.x * SHADE_THREADS + threadIdx.x; i < n; i += gridDim.x * SHADE_THREADS) {
-    const uint32_t pix = A.q_vox[i];
+    uint32_t pix = 0u;
+    if (i < nq) {
+      pix = A.q_vox[i];
+    } else {  // walked again (k_primary_walk)
+      pix = A.q_walk[i - nq];
+      if ((pix & WALKED_VOXEL) == 0u) continue;
+      pix &= ~WALKED_VOXEL;
+    }
     const PrimaryCtx c = primary_ctx(s, pix % A.iw, pix / A.iw, A.iw);
     const uint4* src = A.pix_hit + (size_t)pix * 5u;
     const HitGeom g = load_pixhit(s, src);  // t and n as refined by k_shade_prep
@@ -2151,16 +2240,6 @@ __device__ __forceinline__ void trace_query_rays(const Scene& s, QueryShare shar
 }
 
 constexpr int QUERY_THREADS = 32;
-
-// Rays per warp of `n` queries on a GPU that holds `warps` of them: a warp
-// walks its rays' diverging paths one after another (64 rays in 2 warps take
-// twice as long as one ray a warp), so with fewer than 32 rays for every
-// resident warp the rays are spread over all of them, and more than 32 are
-// never taken at once.
-__host__ __device__ __forceinline__ uint32_t query_unit(uint64_t n, uint32_t warps) {
-  const uint64_t u = (n + warps - 1u) / warps;
-  return u < 1u ? 1u : u > 32u ? 32u : (uint32_t)u;
-}
 
 // One warp per block, `unit` rays each.  (The state machine below serves rays
 // by the thousand; for a few rays its turns cost more than they gather:

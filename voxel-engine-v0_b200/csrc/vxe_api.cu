@@ -50,7 +50,7 @@ enum Img {
   IMG_GOD0, IMG_GOD1, IMG_PRE_TAA, IMG_OUTPUT, IMG_OHIST0, IMG_OHIST1, IMG_HITS, IMG_TILE_COUNT, IMG_TILE_SLOTS,
   IMG_PIXHIT, IMG_QVOX, IMG_QFAR, IMG_QCOUNT, IMG_QSHADOW, IMG_QLIGHT, IMG_PXSHADOW, IMG_PXLIGHT,
   IMG_PROBE_RECS, IMG_SLAB_TASKS, IMG_SLAB_RES, IMG_SLAB_HITS, IMG_PXFIRST, IMG_PXPROBE, IMG_PXMASK, IMG_PXTASK,
-  IMG_QPENDING, IMG_GODPRE, IMG_PXGOV,
+  IMG_QPENDING, IMG_GODPRE, IMG_PXGOV, IMG_QWALK,
   IMG_N
 };
 
@@ -99,6 +99,8 @@ struct FrameState {
 // resolve and the voxel shading) and joins back before the godray pass.
 struct SideStream {
   cudaStream_t s = nullptr;
+  cudaStream_t w = nullptr;  // the walks of the pixels the resolve left (k_primary_walk)
+  cudaEvent_t walked = nullptr;
   cudaEvent_t fork = nullptr, mid = nullptr, prep = nullptr, join = nullptr;
   cudaEvent_t pre = nullptr, table = nullptr;  // walk next -> side, grass table ready -> compute
   cudaEvent_t sun_fork = nullptr, sun = nullptr;  // frame start -> side, sun horizon ready -> compute
@@ -304,7 +306,7 @@ constexpr uint32_t kFrameSlabBits = 4;
 // Grass slab marches those probes ask for, per internal pixel.
 constexpr size_t kSlabsPerPixel = 4;
 
-constexpr size_t kQcountBytes = 64 + (size_t)(4096u << (kFrameSlabBits + 1u)) * 4;  // queue counters, then the slab bins
+constexpr size_t kQcountBytes = ((size_t)vxe::dev::QCOUNT_WORDS + (4096u << (kFrameSlabBits + 1u))) * 4;  // queue counters, then the slab bins
 
 size_t img_bytes(const FrameState& F, int i) {
   const size_t in = (size_t)F.iw * F.ih, pn = (size_t)F.pw * F.ph;
@@ -326,6 +328,7 @@ size_t img_bytes(const FrameState& F, int i) {
     case IMG_PIXHIT:
       return in * 80;
     case IMG_QVOX: case IMG_QFAR: case IMG_QSHADOW: case IMG_QLIGHT: case IMG_PXSHADOW: case IMG_QPENDING:
+    case IMG_QWALK:
       return in * 4;
     case IMG_PROBE_RECS:
       return in * kProbesPerPixel * sizeof(vxe::dev::ProbeRec);
@@ -645,6 +648,7 @@ void frame_fill(vxe_ctx* c, FrameState& F, const vxe_camera_gpu& cam, FrameArgs&
   // the wavefront walk leaves grass-voxel blade marches to k_slab_eval
   A.px_gov = (c->flags & VXE_FLAG_PRIMARY_MEGAKERNEL) ? nullptr : (uint4*)S->img[IMG_PXGOV].p;
   A.q_pending = (uint32_t*)S->img[IMG_QPENDING].p;
+  A.q_walk = (uint32_t*)S->img[IMG_QWALK].p;
   A.god_pre = (c->flags & VXE_FLAG_PRIMARY_MEGAKERNEL) ? nullptr : (float4*)S->img[IMG_GODPRE].p;
   A.god_tag = ++c->god_tag ? c->god_tag : ++c->god_tag;  // never 0, what the buffers start with
 }
@@ -654,7 +658,8 @@ void frame_fill(vxe_ctx* c, FrameState& F, const vxe_camera_gpu& cam, FrameArgs&
 vxe_status side_ready(vxe_ctx* c, SideStream& S) {
   if (S.s) return VXE_OK;
   CK(cudaStreamCreateWithFlags(&S.s, cudaStreamNonBlocking));
-  for (cudaEvent_t* e : {&S.fork, &S.mid, &S.prep, &S.join, &S.pre, &S.table, &S.sun_fork, &S.sun})
+  CK(cudaStreamCreateWithFlags(&S.w, cudaStreamNonBlocking));
+  for (cudaEvent_t* e : {&S.walked, &S.fork, &S.mid, &S.prep, &S.join, &S.pre, &S.table, &S.sun_fork, &S.sun})
     CK(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
   return VXE_OK;
 }
@@ -664,7 +669,11 @@ void side_release(SideStream& S) {
     cudaStreamSynchronize(S.s);
     cudaStreamDestroy(S.s);
   }
-  for (cudaEvent_t e : {S.fork, S.mid, S.prep, S.join, S.pre, S.table, S.sun_fork, S.sun})
+  if (S.w) {
+    cudaStreamSynchronize(S.w);
+    cudaStreamDestroy(S.w);
+  }
+  for (cudaEvent_t e : {S.walked, S.fork, S.mid, S.prep, S.join, S.pre, S.table, S.sun_fork, S.sun})
     if (e) cudaEventDestroy(e);
   S = SideStream{};
 }
@@ -701,6 +710,7 @@ vxe_status frame_enqueue(vxe_ctx* c, FrameState& F, const FrameArgs& A, bool tim
       return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((threads + SHADE_THREADS - 1) / SHADE_THREADS,
                                                                 (uint64_t)c->shade_wave));
     };
+    auto walk_grid = [&](uint64_t pixels) { return (unsigned)std::min<uint64_t>(pixels, (uint64_t)c->shade_wave); };
     CK(cudaMemsetAsync(A.q_count, 0, kQcountBytes, st));
     if (table_side) CK(cudaEventRecord(side->pre, st));
     if (timed) CK(cudaEventRecord(F.ev[7], st));
@@ -733,6 +743,11 @@ vxe_status frame_enqueue(vxe_ctx* c, FrameState& F, const FrameArgs& A, bool tim
       CK(cudaEventRecord(side->mid, st));
       CK(cudaStreamWaitEvent(side->s, side->mid, 0));
       k_shade_far<1><<<grid(npix), SHADE_THREADS, 0, side->s>>>(A);
+      CK(cudaStreamWaitEvent(side->w, side->mid, 0));
+      k_primary_walk<<<walk_grid(npix), WALK_THREADS, 0, side->w>>>(A);
+      CK(cudaEventRecord(side->walked, side->w));
+    } else {
+      k_primary_walk<<<walk_grid(npix), WALK_THREADS, 0, st>>>(A);
     }
     k_shade_prep<<<grid(npix), SHADE_THREADS, 0, st>>>(A);
     k_shade_refine<<<grid(npix), SHADE_THREADS, 0, st>>>(A);
@@ -742,13 +757,17 @@ vxe_status frame_enqueue(vxe_ctx* c, FrameState& F, const FrameArgs& A, bool tim
       // writes: it runs beside the rest of the voxel shading.
       CK(cudaEventRecord(side->prep, st));
       CK(cudaStreamWaitEvent(side->s, side->prep, 0));
+      CK(cudaStreamWaitEvent(side->s, side->walked, 0));
       if (timed) CK(cudaEventRecord(F.ev[4], side->s));
       k_godray<<<dim3((F.iw + POST_THREADS_X - 1) / POST_THREADS_X, (F.ih + POST_THREADS_Y - 1) / POST_THREADS_Y),
                  dim3(POST_THREADS_X, POST_THREADS_Y), 0, side->s>>>(A);
       if (timed) CK(cudaEventRecord(F.ev[5], side->s));
       CK(cudaEventRecord(side->join, side->s));
     }
-    if (side) CK(cudaStreamWaitEvent(st, side->sun, 0));
+    if (side) {
+      CK(cudaStreamWaitEvent(st, side->walked, 0));
+      CK(cudaStreamWaitEvent(st, side->sun, 0));
+    }
     k_shade_shadow<<<grid(npix), SHADE_THREADS, 0, st>>>(A);
     k_shade_lights<<<grid((uint64_t)npix * 8u), SHADE_THREADS, 0, st>>>(A);
     k_shade_vox<<<grid(npix), SHADE_THREADS, 0, st>>>(A);
@@ -809,13 +828,18 @@ vxe_status views_enqueue(vxe_ctx* c, const vxe::dev::FrameArgsViews& V, uint32_t
   CK(cudaEventRecord(side->mid, st));
   CK(cudaStreamWaitEvent(side->s, side->mid, 0));
   k_shade_far_views<1><<<grid(max_pix), SHADE_THREADS, 0, side->s>>>(V);
+  CK(cudaStreamWaitEvent(side->w, side->mid, 0));
+  k_primary_walk_views<<<dim3((unsigned)std::min<uint64_t>(max_pix, per_view), 1, n), WALK_THREADS, 0, side->w>>>(V);
+  CK(cudaEventRecord(side->walked, side->w));
   k_shade_prep_views<<<grid(max_pix), SHADE_THREADS, 0, st>>>(V);
   k_shade_refine_views<<<grid(max_pix), SHADE_THREADS, 0, st>>>(V);
   CK(cudaEventRecord(side->prep, st));
   CK(cudaStreamWaitEvent(side->s, side->prep, 0));
+  CK(cudaStreamWaitEvent(side->s, side->walked, 0));
   k_godray_views<<<dim3((max_iw + POST_THREADS_X - 1) / POST_THREADS_X, (max_ih + POST_THREADS_Y - 1) / POST_THREADS_Y, n),
                    dim3(POST_THREADS_X, POST_THREADS_Y), 0, side->s>>>(V);
   CK(cudaEventRecord(side->join, side->s));
+  CK(cudaStreamWaitEvent(st, side->walked, 0));
   CK(cudaStreamWaitEvent(st, side->sun, 0));
   k_shade_shadow_views<<<grid(max_pix), SHADE_THREADS, 0, st>>>(V);
   k_shade_lights_views<<<grid(max_pix * 8u), SHADE_THREADS, 0, st>>>(V);
@@ -1607,10 +1631,10 @@ vxe_status vxe_get_frame_stats(vxe_ctx* c, vxe_frame_stats* out) {
   if (!c->fr.img[IMG_QCOUNT].p || (c->flags & VXE_FLAG_PRIMARY_MEGAKERNEL)) return VXE_OK;
   cudaSetDevice(c->device);
   CK(cudaStreamSynchronize(c->compute));
-  uint32_t q[16];
+  uint32_t q[vxe::dev::QCOUNT_WORDS];
   CK(cudaMemcpy(q, c->fr.img[IMG_QCOUNT].p, sizeof q, cudaMemcpyDeviceToHost));
-  out->voxel_pixels = q[0];
-  out->far_pixels = q[1];
+  out->voxel_pixels = q[0] + q[16];  // with the pixels walked again
+  out->far_pixels = q[1] + q[17];
   out->probes = q[4];
   out->pending_pixels = q[5];
   out->slab_tasks = q[6] - q[12];  // without the marches the walk left open

@@ -241,16 +241,6 @@ __global__ void __launch_bounds__(TILE_THREADS) k_batch_tiles(const __grid_const
 
 __device__ __forceinline__ void store_rec_at(uint4* out, size_t i, const HitRec& h) { store_rec(out + i * 2u, h); }
 
-// Appends `value` to queue q; the lanes that arrive together share one atomic.
-__device__ __forceinline__ void enqueue_active(uint32_t* q, uint32_t* counter, uint32_t value) {
-  const uint32_t mask = __activemask();
-  const uint32_t lane = threadIdx.x & 31u, leader = __ffs(mask) - 1u;
-  uint32_t base = 0u;
-  if (lane == leader) base = atomicAdd(counter, (uint32_t)__popc(mask));
-  base = __shfl_sync(mask, base, leader);
-  q[base + (uint32_t)__popc(mask & ((1u << lane) - 1u))] = value;
-}
-
 __device__ __forceinline__ void store_hitgeom(uint4* dst, const HitGeom& g) {
   dst[0] = make_uint4(__float_as_uint(g.t), __float_as_uint(g.n.x), __float_as_uint(g.n.y), __float_as_uint(g.n.z));
   dst[1] = make_uint4(__float_as_uint(g.root_bmin.x), __float_as_uint(g.root_bmin.y), __float_as_uint(g.root_bmin.z),
@@ -509,7 +499,7 @@ __global__ void __launch_bounds__(BATCH_THREADS, SLAB_MIN_BLOCKS) k_batch_slab_e
   __shared__ SlabWarp work[BATCH_THREADS / 32];
   const uint32_t n_reqs = B.hdr->n_reqs;
   const uint32_t n = min(B.dcount[2], B.slab_cap), warps = gridDim.x * (BATCH_THREADS / 32);
-  const uint32_t chunk = n >= warps * SLAB_CHUNK ? SLAB_CHUNK : 32u;
+  const uint32_t chunk = n >= warps * (SLAB_CHUNK / 2u) ? SLAB_CHUNK : 32u;  // few tasks: over all the warps
   for (uint32_t i = blockIdx.x * (BATCH_THREADS / 32) + (threadIdx.x >> 5); i * chunk < n; i += warps) {
     slab_march_chunk(
         work[threadIdx.x >> 5], i * chunk, chunk, n,
@@ -624,7 +614,7 @@ __global__ void __launch_bounds__(BATCH_THREADS) k_batch_resolve(const __grid_co
 }
 
 // Rays whose answer is a grass voxel: most refinement marches miss at once
-// and are written here; the rest march one lane each in k_batch_refine.
+// and are written here; the rest march in k_batch_refine.
 __global__ void __launch_bounds__(BATCH_THREADS) k_batch_refine_list(const __grid_constant__ BatchArgs B) {
   const uint32_t n_reqs = B.hdr->n_reqs;
   const uint32_t n = B.dcount[4];
@@ -644,15 +634,35 @@ __global__ void __launch_bounds__(BATCH_THREADS) k_batch_refine_list(const __gri
   }
 }
 
-__global__ void __launch_bounds__(BATCH_THREADS, SLAB_MIN_BLOCKS) k_batch_refine(const __grid_constant__ BatchArgs B) {
+__global__ void __launch_bounds__(MARCH_THREADS) k_batch_refine(const __grid_constant__ BatchArgs B) {
+  extern __shared__ MarchBlock march_shared[];
+  MarchBlock& M = march_shared[0];
+  march_tapers(M);
   const uint32_t n_reqs = B.hdr->n_reqs;
-  const uint32_t n = B.dcount[7];
-  for (uint32_t i = blockIdx.x * BATCH_THREADS + threadIdx.x; i < n; i += gridDim.x * BATCH_THREADS) {
-    const uint32_t ray = B.q_pending[i];
-    const BatchRay br = batch_ray(B, n_reqs, ray);
-    const Scene s = batch_scene(B, &B.cams[br.q->cam]);
-    const HitGeom best = load_pixhit(s, B.px_hit + (size_t)ray * 4u);
-    store_rec_at(br.q->out, (size_t)br.gy * br.q->w + br.gx, viewport_voxel_rec(s, br.gx, br.gy, best));
+  const uint32_t n = B.dcount[7], warps = gridDim.x * (MARCH_THREADS / 32);
+  const uint32_t chunk = n >= warps * (MARCH_CHUNK / 4u) ? MARCH_CHUNK : 32u;  // few marches: over all the warps
+  Scene s;
+  auto load = [&](uint32_t j, const BatchRay& br, v3* ro, v3* rd) {
+    s = batch_scene(B, &B.cams[br.q->cam]);
+    *ro = cam_pos(s);
+    *rd = ray_dir_from_pixel(s, V2((float)br.gx + 0.5f, (float)br.gy + 0.5f));
+    return load_pixhit(s, B.px_hit + (size_t)B.q_pending[j] * 4u);
+  };
+  for (uint32_t i = blockIdx.x * (MARCH_THREADS / 32) + (threadIdx.x >> 5); i * chunk < n; i += warps) {
+    grass_march_chunk(
+        M.warp[threadIdx.x >> 5], M.taper, i * chunk, chunk, n,
+        [&](uint32_t j, v3* ro, v3* rd, v2* iv, GrassCell* c) -> const Scene& {
+          const HitGeom best = load(j, batch_ray(B, n_reqs, B.q_pending[j]), ro, rd);
+          grass_refine_setup(s, *ro, *rd, best, c, iv);
+          return s;
+        },
+        [&](uint32_t j, bool hit, float t, v3 nrm) {
+          const BatchRay br = batch_ray(B, n_reqs, B.q_pending[j]);
+          v3 ro, rd;
+          HitGeom best = load(j, br, &ro, &rd);
+          if (hit) { best.t = t; best.n = nrm; }
+          store_rec_at(br.q->out, (size_t)br.gy * br.q->w + br.gx, make_rec(best, ro, rd, vs_(s), true));
+        });
   }
 }
 

@@ -1002,6 +1002,16 @@ __device__ __forceinline__ void enqueue(uint32_t* q, uint32_t* counter, bool min
   q[base + __popc(mask & ((1u << lane) - 1u))] = value;
 }
 
+// Appends `value` to queue q; the lanes that arrive together share one atomic.
+__device__ __forceinline__ void enqueue_active(uint32_t* q, uint32_t* counter, uint32_t value) {
+  const uint32_t mask = __activemask();
+  const uint32_t lane = threadIdx.x & 31u, leader = __ffs(mask) - 1u;
+  uint32_t base = 0u;
+  if (lane == leader) base = atomicAdd(counter, (uint32_t)__popc(mask));
+  base = __shfl_sync(mask, base, leader);
+  q[base + (uint32_t)__popc(mask & ((1u << lane) - 1u))] = value;
+}
+
 __device__ __forceinline__ uint32_t warp_uniform_end(uint32_t n) { return (n + 31u) & ~31u; }
 
 // Walk summary of a pixel that met probes (px_probe.x): probes met (24 bits),
@@ -1189,7 +1199,7 @@ __device__ __forceinline__ void k_slab_eval_body(const FrameArgs& A) {
   __shared__ SlabWarp work[SHADE_THREADS / 32];
   const Scene s = make_scene(A, false);
   const uint32_t n = min(A.q_count[6], A.slab_cap), warps = gridDim.x * (SHADE_THREADS / 32);
-  const uint32_t chunk = n >= warps * SLAB_CHUNK ? SLAB_CHUNK : 32u;  // few tasks: over all the warps
+  const uint32_t chunk = n >= warps * (SLAB_CHUNK / 2u) ? SLAB_CHUNK : 32u;  // few tasks: over all the warps
   for (uint32_t i = blockIdx.x * (SHADE_THREADS / 32) + (threadIdx.x >> 5); i * chunk < n; i += warps) {
     slab_march_chunk(
         work[threadIdx.x >> 5], i * chunk, chunk, n,
@@ -1449,34 +1459,60 @@ __global__ void __launch_bounds__(SHADE_THREADS, SHADE_MIN_BLOCKS) k_shade_prep_
   k_shade_prep_body(V.v[blockIdx.z]);
 }
 
-// The refinement marches, one lane each: a quarter of the voxel pixels march,
-// and inside k_shade_prep they held 4.8 of 32 lanes for 70 % of its time.
-// With slab_push's atomics without results: 1080p frame 3.66 -> 3.54 ms,
-// 256x144 frame 0.54 -> 0.51 ms, the 64-request batch 63 -> 59 ms.
+// The refinement marches (grass_march_chunk): a quarter of the voxel pixels
+// march, and inside k_shade_prep those marches held 4.8 of 32 lanes for 70 %
+// of its time; one lane each, 9.9.
+constexpr int MARCH_THREADS = 128;
+struct MarchBlock {  // dynamic shared memory of the march kernels
+  MarchWarp warp[MARCH_THREADS / 32];
+  float taper[GRASS_TAPER_N];  // 3 lods x 6 segments
+};
+__device__ __forceinline__ void march_tapers(MarchBlock& M) {
+  if (threadIdx.x < GRASS_TAPER_N) {
+    const uint32_t lod = threadIdx.x / 6u, sg = threadIdx.x % 6u, segs = grass_lod_segs(lod);
+    M.taper[threadIdx.x] = sg < segs ? grass_taper_value(1.0f / fmax_((float)segs, 1.0f), sg) : 0.0f;
+  }
+  __syncthreads();
+}
 __device__ __forceinline__ void k_shade_refine_body(const FrameArgs& A) {
+  extern __shared__ MarchBlock march_shared[];
+  MarchBlock& M = march_shared[0];
+  const uint32_t n = A.q_count[14], warps = gridDim.x * (MARCH_THREADS / 32);
+  const uint32_t chunk = n >= warps * (MARCH_CHUNK / 4u) ? MARCH_CHUNK : 32u;  // few marches: over all the warps
+  if (blockIdx.x * (MARCH_THREADS / 32) * chunk >= n) return;
+  march_tapers(M);
   const Scene s = make_scene(A, false);
-  const uint32_t n = A.q_count[14], end = warp_uniform_end(n);
-  for (uint32_t i = blockIdx.x * SHADE_THREADS + threadIdx.x; i < end; i += gridDim.x * SHADE_THREADS) {
-    bool fresh = false, light = false;
-    uint32_t pix = 0u;
-    if (i < n) {
-      pix = A.q_pending[i];
-      const PrimaryCtx c = primary_ctx(s, pix % A.iw, pix / A.iw, A.iw);
-      uint4* src = A.pix_hit + (size_t)pix * 5u;
-      HitGeom g = load_pixhit(s, src);
-      if (grass_refine(s, c, g)) {
-        profile_add(A, PROFILE_GRASS, 1u);
-        src[0] = make_uint4(__float_as_uint(g.t), __float_as_uint(g.n.x), __float_as_uint(g.n.y),
-                            __float_as_uint(g.n.z));
-      }
-      shade_classify(A, s, c, g, &fresh, &light);
-    }
-    enqueue(A.q_shadow, &A.q_count[2], fresh, pix);
-    enqueue(A.q_light, &A.q_count[3], light, pix);
+  for (uint32_t i = blockIdx.x * (MARCH_THREADS / 32) + (threadIdx.x >> 5); i * chunk < n; i += warps) {
+    grass_march_chunk(
+        M.warp[threadIdx.x >> 5], M.taper, i * chunk, chunk, n,
+        [&](uint32_t j, v3* ro, v3* rd, v2* iv, GrassCell* cell) -> const Scene& {
+          const uint32_t pix = A.q_pending[j];
+          const PrimaryCtx c = primary_ctx(s, pix % A.iw, pix / A.iw, A.iw);
+          *ro = c.ro;
+          *rd = c.rd;
+          grass_refine_setup(s, c.ro, c.rd, load_pixhit(s, A.pix_hit + (size_t)pix * 5u), cell, iv);
+          return s;
+        },
+        [&](uint32_t j, bool hit, float t, v3 nrm) {
+          const uint32_t pix = A.q_pending[j];
+          uint4* src = A.pix_hit + (size_t)pix * 5u;
+          HitGeom g = load_pixhit(s, src);
+          if (hit) {
+            profile_add(A, PROFILE_GRASS, 1u);
+            g.t = t;
+            g.n = nrm;
+            src[0] = make_uint4(__float_as_uint(g.t), __float_as_uint(g.n.x), __float_as_uint(g.n.y),
+                                __float_as_uint(g.n.z));
+          }
+          bool fresh, light;
+          shade_classify(A, s, primary_ctx(s, pix % A.iw, pix / A.iw, A.iw), g, &fresh, &light);
+          if (fresh) enqueue_active(A.q_shadow, &A.q_count[2], pix);
+          if (light) enqueue_active(A.q_light, &A.q_count[3], pix);
+        });
   }
 }
-__global__ void __launch_bounds__(SHADE_THREADS, SLAB_MIN_BLOCKS) k_shade_refine(const __grid_constant__ FrameArgs A) { k_shade_refine_body(A); }
-__global__ void __launch_bounds__(SHADE_THREADS, SLAB_MIN_BLOCKS) k_shade_refine_views(const __grid_constant__ FrameArgsViews V) {
+__global__ void __launch_bounds__(MARCH_THREADS) k_shade_refine(const __grid_constant__ FrameArgs A) { k_shade_refine_body(A); }
+__global__ void __launch_bounds__(MARCH_THREADS) k_shade_refine_views(const __grid_constant__ FrameArgsViews V) {
   k_shade_refine_body(V.v[blockIdx.z]);
 }
 

@@ -678,6 +678,13 @@ void side_release(SideStream& S) {
   S = SideStream{};
 }
 
+// Blocks of the march kernels for up to `marches` of them: what the GPU holds
+// of their shared memory (4 blocks per SM), in chunks of 32 or 64 per warp.
+unsigned march_grid(const vxe_ctx* c, uint64_t marches) {
+  const uint64_t wave = (uint64_t)c->shade_wave / 4u;  // shade_wave: 16 blocks per SM
+  return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(marches / 128u + 1u, wave));
+}
+
 // `table_side`: A reads the grass cell table, which is made current here, on
 // the side stream beside the walk.
 vxe_status frame_enqueue(vxe_ctx* c, FrameState& F, const FrameArgs& A, bool timed, cudaStream_t st,
@@ -750,7 +757,7 @@ vxe_status frame_enqueue(vxe_ctx* c, FrameState& F, const FrameArgs& A, bool tim
       k_primary_walk<<<walk_grid(npix), WALK_THREADS, 0, st>>>(A);
     }
     k_shade_prep<<<grid(npix), SHADE_THREADS, 0, st>>>(A);
-    k_shade_refine<<<grid(npix), SHADE_THREADS, 0, st>>>(A);
+    k_shade_refine<<<march_grid(c, npix), MARCH_THREADS, sizeof(MarchBlock), st>>>(A);
     if (side) {
       // Every depth is final here (voxel pixels' from k_shade_prep and k_shade_refine, far
       // pixels' from k_shade_far), and godray reads nothing else the shading
@@ -832,7 +839,7 @@ vxe_status views_enqueue(vxe_ctx* c, const vxe::dev::FrameArgsViews& V, uint32_t
   k_primary_walk_views<<<dim3((unsigned)std::min<uint64_t>(max_pix, per_view), 1, n), WALK_THREADS, 0, side->w>>>(V);
   CK(cudaEventRecord(side->walked, side->w));
   k_shade_prep_views<<<grid(max_pix), SHADE_THREADS, 0, st>>>(V);
-  k_shade_refine_views<<<grid(max_pix), SHADE_THREADS, 0, st>>>(V);
+  k_shade_refine_views<<<dim3(std::max(1u, march_grid(c, max_pix) / n), 1, n), MARCH_THREADS, sizeof(MarchBlock), st>>>(V);
   CK(cudaEventRecord(side->prep, st));
   CK(cudaStreamWaitEvent(side->s, side->prep, 0));
   CK(cudaStreamWaitEvent(side->s, side->walked, 0));
@@ -1064,6 +1071,10 @@ vxe_status vxe_create(const vxe_config* cfg, vxe_ctx** out) {
     const vxe_status sb = stage_block_add(c);
     if (sb != VXE_OK) return bail(sb);
   }
+  for (const void* k : {(const void*)vxe::dev::k_shade_refine, (const void*)vxe::dev::k_shade_refine_views,
+                        (const void*)vxe::dev::k_batch_refine})
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(vxe::dev::MarchBlock)) != cudaSuccess)
+      return bail(VXE_ERR_DEVICE);
   *out = c;
   return VXE_OK;
 }
@@ -2154,7 +2165,7 @@ vxe_status launch_persistent(vxe_ctx* c, BatchLane& L, const BatchArgs& B, bool 
     k_batch_slab_pick<<<c->shade_wave, BATCH_THREADS, 0, L.stream>>>(B);
     k_batch_resolve<<<c->shade_wave, BATCH_THREADS, 0, L.stream>>>(B);
     k_batch_refine_list<<<c->shade_wave, BATCH_THREADS, 0, L.stream>>>(B);
-    k_batch_refine<<<c->shade_wave, BATCH_THREADS, 0, L.stream>>>(B);
+    k_batch_refine<<<march_grid(c, ~0ull), MARCH_THREADS, sizeof(MarchBlock), L.stream>>>(B);
     k_batch_far<<<c->shade_wave, BATCH_THREADS, 0, L.stream>>>(B);
     if (sorted) CK(cudaStreamWaitEvent(L.stream, L.side.join, 0));
   }

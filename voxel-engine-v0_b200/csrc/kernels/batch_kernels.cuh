@@ -87,7 +87,7 @@ struct BatchArgs {
   uint32_t slab_bits;             // SlabSink::bits
   uint32_t ray_cap;               // per-ray arrays' capacity
   unsigned long long* px_first;
-  uint32_t* px_task;
+  uint32_t* px_task;              // until k_batch_slab_pick: the rays whose walks left a march open, dcount[9]
   uint2* px_mask;
   uint2* px_probe;
   uint4* px_hit;                  // 4 x uint4 per ray: voxel answer of a ray that met probes or needs refining
@@ -97,7 +97,8 @@ struct BatchArgs {
                                   // on in q_pending
   uint32_t* q_far;                // rays without a voxel answer (heightfield)
   uint32_t* dcount;               // [0] probes, [1] pending rays, [2] slab tasks, [3] slab hits, [4] refine, [5] far,
-                                  // [6] bin positions given out, [7] refinement marches; from [16] the slab bins
+                                  // [6] bin positions given out, [7] refinement marches, [9] marches left open; from
+                                  // [16] the slab bins
   // coherent queries: query rays binned by (origin chunk, direction octant)
   uint32_t* q_keys;               // bin of each query ray
   uint32_t* q_perm;               // query rays in bin order
@@ -297,6 +298,7 @@ __device__ __forceinline__ void batch_item(const BatchArgs& B, const BatchHeader
         const uint32_t stored = ph.seq > 0xFFFFFFu ? 0u : ph.recorded;
         B.px_probe[ray] = make_uint2(probe_summary(ph.seq, ph.best_cand, ph.phase, ph.first_phase == 0u, vox), stored);
         enqueue_active(B.q_pending, &B.dcount[1], ray);
+        if (vox && vt.gov_state == 1u) enqueue_active(B.px_task, &B.dcount[9], ray);  // (k_batch_slab_pick fills it)
       } else {
         batch_finish(B, s, q, ray, gx, gy, vox, vt.best);
       }
@@ -441,11 +443,10 @@ __global__ void __launch_bounds__(BATCH_THREADS) k_batch_probe_dda(const __grid_
     if (lost) atomicMin(&B.px_probe[r.pixel].y, 0u);
   }
   // the blade marches the walks left open
-  const uint32_t np = B.dcount[1];
+  const uint32_t np = B.dcount[9];
   for (uint32_t i = blockIdx.x * BATCH_THREADS + threadIdx.x; i < np; i += gridDim.x * BATCH_THREADS) {
-    const uint32_t ray = B.q_pending[i];
+    const uint32_t ray = B.px_task[i];
     const uint4 gv = B.px_gov[ray];
-    if (gv.x != 1u) continue;
     const BatchRay br = batch_ray(B, n_reqs, ray);
     const Scene s = batch_scene(B, &B.cams[br.q->cam]);
     const uint4 h = B.px_hit[(size_t)ray * 4u];

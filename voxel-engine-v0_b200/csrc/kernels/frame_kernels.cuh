@@ -66,10 +66,11 @@ struct FrameArgs {
   uint32_t* q_count;  // [0] voxel, [1] far, [2] fresh shadow, [3] light gather, [4] probes, [5] pending,
                       // [6] slab tasks, [7] slab hits, [8] far pixels queued by the walk, [11] bin positions
                       // given out, [12] / [13] the gov tasks / hits among [6] / [7], [14] refinement marches,
-                      // [15] pixels to walk again, [16] / [17] of them: voxel / far answers; from
-                      // QCOUNT_WORDS on the slab bins
+                      // [15] pixels to walk again, [16] / [17] of them: voxel / far answers,
+                      // [20] marches the walk left open; from QCOUNT_WORDS on the slab bins
   uint32_t* q_shadow;  // voxel pixels that trace a fresh sun shadow this frame
-  uint32_t* q_light;   // voxel pixels that gather local lights
+  uint32_t* q_light;   // voxel pixels that gather local lights; until the probes are done, the pixels whose
+                       // grass-voxel march the walk left open (q_count[20])
   float* px_shadow;    // fresh sun transmittance per pixel (q_shadow pixels)
   float4* px_light;    // light gather result per pixel (q_light pixels)
   // deferred grass column probes (PROBE_RECORD -> k_probe_dda -> k_slab_eval
@@ -1035,11 +1036,13 @@ __device__ __forceinline__ unsigned long long slab_key(uint32_t phase, float t, 
 // The end of a pixel's walk in record mode: the voxel answer's PixHit, and
 // for pixels that met probes the walk summary (the rest is final).
 __device__ __forceinline__ void walk_finish(const FrameArgs& A, uint32_t pix, const VoxTraceResult& vt,
-                                            const ProbeHook& ph, uint32_t tile_count, bool* vox, bool* pend) {
+                                            const ProbeHook& ph, uint32_t tile_count, bool* vox, bool* pend,
+                                            bool* gov) {
   *vox = vt.in_grid && vt.best.hit != 0u;
   if (*vox) store_pixhit(A.pix_hit + (size_t)pix * 5u, vt.best, vt);
   const uint32_t gs = *vox ? vt.gov_state : 0u;
   *pend = ph.seq != 0u || gs != 0u;
+  *gov = gs == 1u;
   if (*pend) {
     A.px_first[pix] = ~0ull;  // no probe hit yet
     A.px_mask[pix] = make_uint2(0u, 0u);
@@ -1080,19 +1083,20 @@ __device__ __forceinline__ void k_primary_trace_body(const FrameArgs& A) {
   stage_tiles(s, A, cslot, cmeta, ccount);
   uint32_t t, gx, gy;
   const bool active = block_pixel(A, &t, &gx, &gy);
-  bool vox = false, pend = false, full = false;
+  bool vox = false, pend = false, gov = false, full = false;
   uint32_t pix = 0u;
   if (active) {
     const PrimaryCtx c = primary_ctx(s, gx, gy, A.iw);
     pix = (uint32_t)c.pix;
     ProbeHook ph = probe_hook_record(A, pix);
     const VoxTraceResult vt = primary_trace_inl<PROBE_RECORD>(s, A, c, cslot[t], cmeta[t], ccount[t], ph);
-    walk_finish(A, pix, vt, ph, ccount[t], &vox, &pend);
+    walk_finish(A, pix, vt, ph, ccount[t], &vox, &pend, &gov);
     full = ph.first_phase <= 1u && ph.phase == 1u;
   }
   enqueue(A.q_vox, &A.q_count[0], active && vox && !pend, pix);
   enqueue(A.q_far, &A.q_count[1], active && !vox && !pend, pix);
   enqueue(A.q_pending, &A.q_count[5], active && pend, pix);
+  enqueue(A.q_light, &A.q_count[20], active && gov, pix);  // (the light gathers' queue is filled later)
   const uint32_t nfull = __popc(__ballot_sync(0xFFFFFFFFu, full));  // frame statistics
   if ((threadIdx.x & 31u) == 0u && nfull != 0u) atomicAdd(&A.q_count[10], nfull);
 }
@@ -1133,14 +1137,15 @@ __device__ __forceinline__ void k_probe_dda_body(const FrameArgs& A) {
   }
   // the blade marches the walk left open are tasks too; one that does not fit
   // leaves its pixel's voxel answer undecided
-  const uint32_t np = A.px_gov ? A.q_count[5] : 0u;
+  // (a queue of their own: found among all pending pixels, one in seven, they
+  // took half of this kernel's time)
+  const uint32_t np = A.q_count[20];
   for (uint32_t i = blockIdx.x * SHADE_THREADS + threadIdx.x; i < np; i += gridDim.x * SHADE_THREADS) {
-    const uint32_t pix = A.q_pending[i];
+    const uint32_t pix = A.q_light[i];
     const uint4 gv = A.px_gov[pix];
-    if (gv.x != 1u) continue;
     const uint4 h = A.pix_hit[(size_t)pix * 5u];
     const PrimaryCtx c = primary_ctx(s, pix % A.iw, pix / A.iw, A.iw);
-    atomicAdd(&A.q_count[12], 1u);
+    atomicAdd(&A.q_count[12], 1u);  // counted among [6] too
     if (!slab_push(sink, slab_gov_task(s, pix, gv.w, c.ro, c.rd, __uint_as_float(h.x),
                                        V3(__uint_as_float(h.y), __uint_as_float(h.z), __uint_as_float(h.w)),
                                        __uint_as_float(gv.y), __uint_as_float(gv.z))))

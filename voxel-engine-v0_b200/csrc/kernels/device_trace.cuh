@@ -2670,7 +2670,56 @@ __device__ __forceinline__ v3 sphere_dir_local(uint32_t i, uint32_t count) {  //
   return V3(cosf_(phi) * r, sinf_(phi) * r, y);
 }
 
-__device__ __noinline__ v4 dda_hit_light(const Scene& s, v3 p0, v3 dir, uint32_t max_steps, float vs) {  // light.wgsl:65-121
+// query_leaf_world for the cell centres of a light ray: the material at p, and
+// for air the cube around p that is air throughout (size 0: none known).
+__device__ __forceinline__ LeafQuery light_cell_query(const Scene& s, v3 p) {
+  const float vs = vs_(s);
+  const float cs = (float)s.cam->chunk_size * vs;
+  const LeafQuery air{p, 0.0f, MAT_AIR};
+  const i3 c = chunk_coord_from_pos(p, cs);
+  const uint32_t slot = grid_lookup_slot(s, c.x, c.y, c.z);
+  if (slot == INVALID || slot >= s.cam->chunk_count) return air;
+  const Meta ch = meta_at(s, slot);
+  const v3 rb = V3((float)ch.ox, (float)ch.oy, (float)ch.oz) * vs;
+  if (ch.macro_base != INVALID) {
+    const float cell = macro_cell_size(cs);
+    const v3 lp = p - rb;
+    if (lp.x < 0.0f || lp.y < 0.0f || lp.z < 0.0f || lp.x >= cs || lp.y >= cs || lp.z >= cs) return air;
+    const int32_t mx = to_i32(floorf(lp.x / cell)), my = to_i32(floorf(lp.y / cell)), mz = to_i32(floorf(lp.z / cell));
+    if (mx < 0 || my < 0 || mz < 0 || mx >= (int32_t)MACRO_DIM || my >= (int32_t)MACRO_DIM || mz >= (int32_t)MACRO_DIM)
+      return air;
+    if (!macro_test(s, ch.macro_base, macro_bit_index((uint32_t)mx, (uint32_t)my, (uint32_t)mz)))
+      return LeafQuery{rb + V3((float)mx, (float)my, (float)mz) * cell, cell, MAT_AIR};
+  }
+  uint32_t idx = ch.node_base;
+  v3 bmin = rb;
+  float size = cs;
+  for (uint32_t d = 0; d < 32; ++d) {
+    const Node n = node_global(s, idx);
+    if (n.child_base == LEAF) return LeafQuery{bmin, size, n.material};
+    if (d >= chunk_max_depth(s)) return LeafQuery{bmin, size, MAT_AIR};
+    const float half = size * 0.5f;
+    const v3 mid = bmin + V3s(half);
+    const float e = 1e-6f * size;
+    const uint32_t hx = p.x > mid.x + e ? 1u : 0u, hy = p.y > mid.y + e ? 1u : 0u, hz = p.z > mid.z + e ? 1u : 0u;
+    const uint32_t ci = hx | (hy << 1) | (hz << 2);
+    const v3 cb = bmin + V3(hx ? half : 0.0f, hy ? half : 0.0f, hz ? half : 0.0f);
+    if ((n.child_mask & (1u << ci)) == 0u) return LeafQuery{cb, half, MAT_AIR};
+    idx = ch.node_base + (n.child_base + child_rank(n.child_mask, ci));
+    bmin = cb;
+    size = half;
+  }
+  return air;
+}
+
+// A light ray visits up to 16 voxel cells, most of them air of the same leaf:
+// a cell whose centre lies in the last air cube is not looked up again.
+// Centres stand half a voxel (0.05 m) from every cube's faces, so the descent
+// from the root could not end elsewhere; beyond 1000 m from the origin, where
+// binary32 steps come near that distance, every cell is looked up.
+// k_shade_lights 742 -> 608 us (1001x601, lights in every chunk), frame 2.96
+// -> 2.86 ms.
+__device__ __forceinline__ v4 dda_hit_light(const Scene& s, v3 p0, v3 dir, uint32_t max_steps, float vs) {  // light.wgsl:65-121
   const v3 gpos = p0 / fmax_(vs, 1e-6f);
   const v3 fl = vfloor(gpos);
   i3 cell{to_i32(fl.x), to_i32(fl.y), to_i32(fl.z)};
@@ -2682,11 +2731,15 @@ __device__ __noinline__ v4 dda_hit_light(const Scene& s, v3 p0, v3 dir, uint32_t
                     fabsf(dir.z) > 1e-6f ? 1.0f / fabsf(dir.z) : 1e30f);
   v3 tMax = V3((nb.x - gpos.x) * inv.x, (nb.y - gpos.y) * inv.y, (nb.z - gpos.z) * inv.z);
   const v3 tDelta = inv;
+  const bool near = fabsf(p0.x) < 1000.0f && fabsf(p0.y) < 1000.0f && fabsf(p0.z) < 1000.0f;
+  LeafQuery air{V3s(0.0f), 0.0f, MAT_AIR};
   for (uint32_t i = 0; i < max_steps; ++i) {
     const v3 c = V3((float)cell.x + 0.5f, (float)cell.y + 0.5f, (float)cell.z + 0.5f) * vs;
-    const LeafQuery lf = query_leaf_world(s, c);
-    if (lf.mat == MAT_LIGHT) return v4{c.x, c.y, c.z, 1.0f};
-    if (lf.mat != MAT_AIR) return v4{0.0f, 0.0f, 0.0f, 0.0f};
+    if (!(near && point_in_cube(c, air.bmin, air.size))) {
+      air = light_cell_query(s, c);
+      if (air.mat == MAT_LIGHT) return v4{c.x, c.y, c.z, 1.0f};
+      if (air.mat != MAT_AIR) return v4{0.0f, 0.0f, 0.0f, 0.0f};
+    }
     if (tMax.x < tMax.y) {
       if (tMax.x < tMax.z) { cell.x += step.x; tMax.x += tDelta.x; }
       else { cell.z += step.z; tMax.z += tDelta.z; }
@@ -2728,8 +2781,9 @@ __device__ __forceinline__ LightFrame light_frame(const Scene& s, v3 hp, v3 n, v
   return F;
 }
 
-__device__ __forceinline__ v3 light_ray_dir(const LightFrame& F, v3 n, uint32_t i) {  // light.wgsl:167-169
-  const v3 sl = normalize(sphere_dir_local(i, LIGHT_RAYS));
+__device__ __forceinline__ v3 light_ray_local(uint32_t i) { return normalize(sphere_dir_local(i, LIGHT_RAYS)); }
+// `sl`: light_ray_local of the ray.
+__device__ __forceinline__ v3 light_ray_dir(const LightFrame& F, v3 n, v3 sl) {  // light.wgsl:167-169
   const v3 ldir = normalize(F.tt * sl.x + F.bb * sl.y + n * sl.z);
   return normalize(rot_about_axis(ldir, n, F.rot));
 }
@@ -2793,7 +2847,7 @@ __device__ __noinline__ v3 gather_voxel_lights(const Scene& s, v3 hp, v3 n, v3 r
   v3 sum = V3s(0.0f);
   if (!lights_possible(s, F.p0)) return light_finish(sum);
   for (uint32_t i = 0; i < LIGHT_RAYS; ++i) {
-    const v4 hit = dda_hit_light(s, F.p0, light_ray_dir(F, n, i), LIGHT_MAX_DIST_VOX, vs_(s));
+    const v4 hit = dda_hit_light(s, F.p0, light_ray_dir(F, n, light_ray_local(i)), LIGHT_MAX_DIST_VOX, vs_(s));
     if (light_accum(s, hp, n, hit, hits, sum)) break;
   }
   return light_finish(sum);

@@ -1590,6 +1590,7 @@ __device__ __forceinline__ void k_shade_lights_body(const FrameArgs& A) {
   const Scene s = make_scene(A, false);
   const uint32_t lane = threadIdx.x & 31u, ray = lane & 7u, group0 = lane & ~7u;
   const uint32_t n = A.q_count[3], groups = n * 8u, end = warp_uniform_end(groups);
+  const v3 sl = light_ray_local(ray);  // the lane's ray in every pixel
   for (uint32_t i = blockIdx.x * SHADE_THREADS + threadIdx.x; i < end; i += gridDim.x * SHADE_THREADS) {
     const bool active = i < groups;
     uint32_t pix = 0u;
@@ -1602,7 +1603,7 @@ __device__ __forceinline__ void k_shade_lights_body(const FrameArgs& A) {
       hp = c.ro + c.rd * g.t;
       nrm = g.n;
       const LightFrame F = light_frame(s, hp, nrm, g.root_bmin);
-      hit = dda_hit_light(s, F.p0, light_ray_dir(F, nrm, ray), LIGHT_MAX_DIST_VOX, vs_(s));
+      hit = dda_hit_light(s, F.p0, light_ray_dir(F, nrm, sl), LIGHT_MAX_DIST_VOX, vs_(s));
     }
     v4 h[LIGHT_RAYS];
     for (uint32_t k = 0; k < LIGHT_RAYS; ++k) {

@@ -155,7 +155,7 @@ struct vxe_ctx {
   // caps on the wavefront's stored grass probes and slab tasks (0: the buffers' sizes)
   uint32_t probe_limit = 0, slab_limit = 0;
   // chunk builder: per-chunk scratch (materials, ground minima, level-5 cell
-  // states and child offsets, solid counts) and events around its two kernels
+  // states and child offsets, solid counts) and events around its kernels
   // asynchronous image reads: a copy stream and one event per ticket slot;
   // out_pending / any_pending: the last output / other image copy not yet
   // waited for by a frame
@@ -1771,7 +1771,7 @@ double cave_s_min(double thr) {
 }  // namespace
 
 namespace {
-// Scratch, events and the two builder kernels on the world-write stream.
+// Scratch, events and the builder kernels on the world-write stream.
 vxe_status build_launch(vxe_ctx* c, vxe::build::BuildArgs& B, uint32_t n) {
   namespace vb = vxe::build;
   // per chunk: materials, level-1 ground minima, level-5 states and child
@@ -1805,6 +1805,10 @@ vxe_status build_launch(vxe_ctx* c, vxe::build::BuildArgs& B, uint32_t n) {
   CK(cudaEventRecord(c->build_ev[1], st));
   vb::k_build_svo<<<n, vb::SVO_THREADS, vb::kStageBytes, st>>>(B);
   CK(cudaGetLastError());
+  if (B.place || B.node_cap) {  // a counting call writes no nodes
+    vb::k_build_ropes<<<n * vb::ROPE_PARTS, vb::ROPE_THREADS, 0, st>>>(B);
+    CK(cudaGetLastError());
+  }
   CK(cudaEventRecord(c->build_ev[2], st));
   c->build_timed = true;
   return VXE_OK;

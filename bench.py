@@ -1027,10 +1027,11 @@ def main():
                         "host buffers; every output lands inside the timed region)",
                 "serial_frame_ms": round(res["e2e"]["serial_seconds"] * 1e3 / args.steps, 3),
                 "device_streaming": device_streaming_line(res["e2e"], args.steps, n)},
-        # per frame: k_grass_wind, k_tiles, k_primary_trace, k_probe_dda, k_slab_eval, k_slab_pick,
-        # k_gov_eval, k_primary_resolve, k_shade_prep, k_shade_shadow, k_shade_lights, k_shade_vox,
-        # k_shade_far x 2 and k_godray_far (side stream), k_godray, k_composite
-        "gpu_launches": 17 * args.steps,
+        # per frame: k_tiles, k_primary_trace, k_grass_wind, k_probe_dda, k_slab_bases, k_slab_order,
+        # k_slab_eval, k_slab_pick, k_primary_resolve, k_primary_walk, k_shade_prep, k_shade_refine,
+        # k_shade_shadow, k_shade_lights, k_shade_vox, k_shade_far x 2, k_sun_tops, k_sun_horizon,
+        # k_godray_far, k_godray, k_composite
+        "gpu_launches": 22 * args.steps,
         "batch": batch,
         "serve": srv,
         "configs": configs,
@@ -1041,11 +1042,14 @@ def main():
     l2 = l2_peak(0)
     prim_s = statistics.mean(res["primary_ms"]) * 1e-3
     trace_s = statistics.mean(res["trace_ms"]) * 1e-3
-    # The reference's voxel trace runs here as five launches (the walk, then the
-    # grass probes' column DDAs, slab marches, pick and resolve); the roofline
-    # unit is that stage, timed by the events around it.
+    # The reference's voxel trace runs here as seven launches (the walk, then the
+    # grass probes' column DDAs, the sort of the slab marches in two launches, the
+    # marches, pick and resolve); the roofline unit is that stage, timed by the
+    # events around it.  The few pixels the stage cannot decide walk again beside
+    # the shading (k_primary_walk), outside these events.
     roof = {"bound": "hbm", "achieved": None, "peak": peak, "unit": "GB/s", "frac": None, "traffic": None,
-            "kernel": "trace stage: k_primary_trace + k_probe_dda + k_slab_eval + k_slab_pick + k_primary_resolve",
+            "kernel": "trace stage: k_primary_trace + k_probe_dda + k_slab_bases + k_slab_order + k_slab_eval + "
+                      "k_slab_pick + k_primary_resolve",
             "peak_kind": peak_kind, "launch_ms": round(trace_s * 1e3, 4),
             "walk_kernel_ms": round(statistics.mean(res["walk_ms"]), 4)}
     present = tuple(int(v) for v in args.present.split("x"))
@@ -1070,7 +1074,7 @@ def main():
                                 "achieved": round(pa, 2), "frac": round(pa / peak, 5),
                                 "algorithmic_bytes_per_frame": ab, "ms": round(prim_s * 1e3, 4)}
     # DRAM bytes of the trace stage per 1080p frame: one ncu capture of the
-    # same five kernels on this workload (data file beside the profiles)
+    # same kernels and k_primary_walk on this workload (data file beside the profiles)
     traffic = REPO / "profiles" / "trace_stage_config2_1080p_dram.json"
     if traffic.exists() and present == (1920, 1080):
         roof["traffic"] = int(json.loads(traffic.read_text())["dram_bytes_per_stage"])

@@ -16,14 +16,12 @@
 //                    whose columns all lie above the surface of a world
 //                    without decorations stores zero rows instead);
 //   k_build_svo      one CTA per chunk: ground min-mip, the cell states of
-//                    levels 4..0 and their scans, the level-5 child offsets
-//                    (16 rounds of one exclusive scan, voxel records written
-//                    as they go), node emission, ropes of levels 0..5
-//                    top-down (one thread per node, its parent found from
-//                    its key), macro bits; a chunk with no solid voxel
-//                    writes its lone air root and returns.
-//   k_build_ropes    ROPE_PARTS CTAs per chunk: the voxels' ropes, eight lanes
-//                    per level-5 node.
+//                    levels 4..0 and their scans, the level-5 child offsets,
+//                    nodes and ropes of levels 0..5 (top-down, one thread per
+//                    node, its parent found from its key), macro bits; a chunk
+//                    with no solid voxel writes its lone air root and returns.
+//   k_build_voxels   VOXEL_PARTS CTAs per chunk: the voxels' nodes and ropes,
+//                    eight lanes per level-5 node.
 //
 // Octree cells.  A cell of level l (0 = the chunk, 6 = a voxel) holds
 // 2^(6-l) voxels per side; its cells are numbered px + pz*S + py*S*S with
@@ -59,10 +57,6 @@ constexpr uint32_t ST_LEAF = 1u << 16;
 constexpr uint32_t ST_FULL = 1u << 17;
 constexpr int SVO_THREADS = 512;
 constexpr int SVO_WARPS = SVO_THREADS / 32;
-// Voxel records of one level-5 round staged in (dynamic) shared memory so
-// they leave as contiguous stores; a round with more writes them directly.
-constexpr uint32_t kStageNodes = 2048u;
-constexpr size_t kStageBytes = kStageNodes * 16u;
 // Shared state words of levels 4..0 (4096 + 512 + 64 + 8 + 1 cells).
 constexpr uint32_t kLowCells = 4681u;
 __host__ __device__ constexpr uint32_t low_off(int l) {
@@ -82,7 +76,7 @@ struct BuildArgs {
   uint8_t* mat;           // n * 64^3 materials
   int32_t* mip1;          // n * 32^2 level-1 ground minima (2x2 columns)
   uint32_t* solid_part;   // n * 16 solid voxel counts, one per column block; k_build_svo leaves the first
-                          // node and the length of the chunk's level-5 list in words 0 and 1 (no ropes to
+                          // node and the length of the chunk's level-5 list in words 0 and 1 (no voxels to
                           // write: length 0)
   uint32_t* st5;          // n * 32^3 level-5 state words
   uint32_t* kb5;          // n * 32^3 level-5 child offsets
@@ -484,13 +478,12 @@ __global__ void __launch_bounds__(SVO_THREADS, 2) k_build_svo(const __grid_const
   __shared__ uint32_t kb[kLowCells];
   __shared__ int32_t mip[kMipWords];
   __shared__ uint32_t ws[SVO_WARPS];
+  __shared__ uint32_t part[16 * SVO_WARPS];  // warp sums of the level-5 rounds
   __shared__ uint32_t K[8];  // K[l]: entries of level l's node list (l = 1..6)
   __shared__ uint32_t bases[8];
-  extern __shared__ uint4 stage[];  // kStageNodes voxel records of one level-5 round
 
   const uint32_t chunk = blockIdx.x, t = threadIdx.x;
   if (chunk >= B.n) return;
-  const uint8_t* mat = B.mat + (size_t)chunk * kVoxels;
   uint32_t* st5 = B.st5 + (size_t)chunk * kCells5;
   uint32_t* kb5 = B.kb5 + (size_t)chunk * kCells5;
   const int32_t chunk_oy = chunk_coord(B, chunk, 1) * kSide;
@@ -607,78 +600,57 @@ __global__ void __launch_bounds__(SVO_THREADS, 2) k_build_svo(const __grid_const
   }
   __syncthreads();
 
-  // -- level-5 child offsets and the voxel list: 16 rounds of 2048 cells, 4
-  // consecutive cells (one row of 8 voxels in x) per thread; each round's
-  // loads are issued before the previous round's scan.  Voxel records go out
-  // as their offsets become known, each one only below node_cap.
+  // -- level-5 child offsets: thread t takes 4 consecutive cells of each of 16
+  // rounds of 2048.  The rounds' warp sums are scanned together, so the block
+  // meets three times and not three times a round; a round's counts and place
+  // within its warp wait in one register.
   const uint32_t cap = B.place ? B.place[chunk].node_count : B.node_cap;
   const size_t first = B.place ? (size_t)B.place[chunk].node_base : (size_t)chunk * cap;
   vxe_node* nodes = B.nodes + first;
   vxe_node_ropes* ropes = B.ropes + first;
-  uint32_t carry = 0;
-  uint4 s4;
-  uint64_t rows[4];  // d = dy * 2 + dz: the 8 voxels (x = 8 * (t & 7) ...) of each row
-  auto load_round = [&](uint32_t r, uint4& sv, uint64_t (&rw)[4]) {
-    const uint32_t c0 = r * 2048u + 4u * t, px0 = c0 & 31u, pz = (c0 >> 5) & 31u, py = c0 >> 10;
-    sv = *reinterpret_cast<const uint4*>(st5 + c0);
+  uint32_t carry;
+  {
+    const uint32_t lane = t & 31u, w = t >> 5;
+    uint32_t pk[16];
 #pragma unroll
-    for (uint32_t d = 0; d < 4u; ++d)
-      rw[d] = *reinterpret_cast<const uint64_t*>(mat + (2u * py + (d >> 1)) * 4096u + (2u * pz + (d & 1u)) * 64u + 2u * px0);
-  };
-  load_round(0, s4, rows);
-#pragma unroll 1
-  for (uint32_t r = 0; r < 16u; ++r) {
-    const uint32_t c0 = r * 2048u + 4u * t, px0 = c0 & 31u, pz = (c0 >> 5) & 31u, py = c0 >> 10;
-    const uint32_t sv[4] = {s4.x, s4.y, s4.z, s4.w};
-    const uint64_t rw[4] = {rows[0], rows[1], rows[2], rows[3]};
-    if (r + 1u < 16u) load_round(r + 1u, s4, rows);
-    uint32_t cnt[4], sum = 0;
+    for (uint32_t r = 0; r < 16u; ++r) {
+      const uint4 s4 = *reinterpret_cast<const uint4*>(st5 + r * 2048u + 4u * t);
+      const uint32_t sv[4] = {s4.x, s4.y, s4.z, s4.w};
+      uint32_t v = 0, c = 0;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      cnt[k] = (sv[k] & ST_MASK) && !(sv[k] & ST_LEAF) ? (uint32_t)__popc(sv[k] & ST_MASK) : 0u;
-      sum += cnt[k];
-    }
-    uint32_t total;
-    const uint32_t round0 = carry;
-    const uint32_t off0 = carry + block_excl_scan(sum, ws, &total);
-    carry += total;
-    const bool staged = total <= kStageNodes;  // block-uniform
-    uint32_t off = off0;
-    uint4 kv;
-    kv.x = off; off += cnt[0];
-    kv.y = off; off += cnt[1];
-    kv.z = off; off += cnt[2];
-    kv.w = off;
-    *reinterpret_cast<uint4*>(kb5 + c0) = kv;
-    uint32_t o = bases[6] + off0;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      if (!cnt[k]) continue;
-#pragma unroll
-      for (int ci = 0; ci < 8; ++ci) {
-        if (!((sv[k] >> ci) & 1u)) continue;
-        const uint32_t cx = 2u * (px0 + k) + (ci & 1), cy = 2u * py + ((ci >> 1) & 1), cz = 2u * pz + ((ci >> 2) & 1);
-        const uint32_t mat_ci =
-            (uint32_t)(rw[((ci >> 1) & 1) * 2 + ((ci >> 2) & 1)] >> (8 * (2 * k + (ci & 1)))) & 0xFFu;
-        const uint4 rec = make_uint4(kInvalid, 0u, mat_ci, cell_key(cx, cy, cz, 6u));
-        if (staged) stage[o - bases[6] - round0] = rec;
-        else if (o < cap) *reinterpret_cast<uint4*>(nodes + o) = rec;
-        ++o;
+      for (int k = 0; k < 4; ++k) {
+        const uint32_t n = (sv[k] & ST_MASK) && !(sv[k] & ST_LEAF) ? (uint32_t)__popc(sv[k] & ST_MASK) : 0u;
+        v += n;
+        c |= n << (12 + 4 * k);
       }
+      uint32_t x = v;
+#pragma unroll
+      for (uint32_t o = 1; o < 32u; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+        if (lane >= o) x += y;
+      }
+      if (lane == 31u) part[r * SVO_WARPS + w] = x;
+      pk[r] = c | (x - v);  // at most 31 * 32 before the lane
     }
-    if (staged) {  // the round's records leave shared memory as one contiguous run
-      __syncthreads();
-      const uint32_t first = bases[6] + round0;
-      for (uint32_t i = t; i < total; i += SVO_THREADS)
-        if (first + i < cap) *reinterpret_cast<uint4*>(nodes + first + i) = stage[i];
-      // the next round's scan barriers order these reads before its stores
+    __syncthreads();
+    const uint32_t o = block_excl_scan(t < 16u * SVO_WARPS ? part[t] : 0u, ws, &carry);
+    if (t < 16u * SVO_WARPS) part[t] = o;
+    __syncthreads();
+#pragma unroll
+    for (uint32_t r = 0; r < 16u; ++r) {
+      uint4 kv;
+      kv.x = part[r * SVO_WARPS + w] + (pk[r] & 0xFFFu);
+      kv.y = kv.x + ((pk[r] >> 12) & 15u);
+      kv.z = kv.y + ((pk[r] >> 16) & 15u);
+      kv.w = kv.z + ((pk[r] >> 20) & 15u);
+      *reinterpret_cast<uint4*>(kb5 + r * 2048u + 4u * t) = kv;
     }
   }
   if (t == 0) {
     K[6] = carry;
     bases[7] = bases[6] + carry;
   }
-  __syncthreads();  // kb5 and the voxel records visible to the CTA
+  __syncthreads();  // kb5 visible to the CTA
   const uint32_t node_count = bases[7];
 
   if (t == 0) write_counts_meta(B, chunk, node_count, solid);
@@ -755,27 +727,33 @@ __global__ void __launch_bounds__(SVO_THREADS, 2) k_build_svo(const __grid_const
   }
 }
 
-// The ropes of level 6 (the voxels: three quarters of a surface chunk's nodes)
-// need only their parents' nodes and ropes, so they are written by as many
-// CTAs as the GPU holds instead of their chunk's one, which waited for three
-// dependent loads per node with 16 warps.  Eight lanes per level-5 node, one
-// per child: the parent's records are read once for all of them and the
-// children's ropes leave as one run.  256 surface and air chunks with their
-// packing: 768 -> 697 us.
-constexpr uint32_t ROPE_PARTS = 8;
-constexpr int ROPE_THREADS = 256;
-__global__ void __launch_bounds__(ROPE_THREADS) k_build_ropes(const __grid_constant__ BuildArgs B) {
-  const uint32_t chunk = blockIdx.x / ROPE_PARTS, part = blockIdx.x % ROPE_PARTS;
+// Level 6 (the voxels: three quarters of a surface chunk's nodes) needs only its
+// parents' nodes and ropes, so it is written by as many CTAs as the GPU holds
+// instead of its chunk's one, which waited for three dependent loads per node
+// with 16 warps and wrote the records between the barriers of its scans.  Eight
+// lanes per level-5 node, one per child: the parent's records are read once
+// for all of them and the children's nodes and ropes leave as one run each.
+// 256 surface and air chunks with the caller's packing: 751 -> 697 us with the
+// ropes here, 662 us with the nodes too and the level-5 scan in one.
+constexpr uint32_t VOXEL_PARTS = 8;
+constexpr int VOXEL_THREADS = 256;
+__global__ void __launch_bounds__(VOXEL_THREADS) k_build_voxels(const __grid_constant__ BuildArgs B) {
+  const uint32_t chunk = blockIdx.x / VOXEL_PARTS, part = blockIdx.x % VOXEL_PARTS;
   const uint32_t lo = B.solid_part[(size_t)chunk * 16u], n = B.solid_part[(size_t)chunk * 16u + 1u];
   const size_t first = B.place ? (size_t)B.place[chunk].node_base : (size_t)chunk * B.node_cap;
-  const vxe_node* nodes = B.nodes + first;
+  const uint8_t* mat = B.mat + (size_t)chunk * kVoxels;
+  vxe_node* nodes = B.nodes + first;
   vxe_node_ropes* ropes = B.ropes + first;
   const bool vec = ((uintptr_t)ropes & 15u) == 0u;
-  for (uint32_t i = part * ROPE_THREADS + threadIdx.x; i < 8u * n; i += ROPE_PARTS * ROPE_THREADS) {
+  for (uint32_t i = part * VOXEL_THREADS + threadIdx.x; i < 8u * n; i += VOXEL_PARTS * VOXEL_THREADS) {
     const uint32_t ci = i & 7u, p = lo + (i >> 3);
     const vxe_node pn = nodes[p];
     if (!(pn.child_mask & (1u << ci))) continue;  // a leaf's mask is 0
+    const uint32_t x = 2u * (pn.key & 63u) + (ci & 1u), y = 2u * ((pn.key >> 6) & 63u) + ((ci >> 1) & 1u),
+                   z = 2u * ((pn.key >> 12) & 63u) + (ci >> 2);
     const uint32_t k = pn.child_base + (uint32_t)__popc(pn.child_mask & ((1u << ci) - 1u));
+    *reinterpret_cast<uint4*>(nodes + k) =
+        make_uint4(kInvalid, 0u, mat[y * 4096u + z * 64u + x], cell_key(x, y, z, 6u));
     store_ropes(ropes + k, child_ropes(nodes, pn, ropes[p], ci), vec);
   }
 }

@@ -296,17 +296,6 @@ __device__ __noinline__ LeafQuery query_leaf_at(const Scene& s, v3 p, v3 root_bm
   return LeafQuery{bmin, size, MAT_AIR};
 }
 
-__device__ __noinline__ LeafQuery query_leaf_world(const Scene& s, v3 p) {  // svo_query.wgsl:270-291
-  const float vs = vs_(s);
-  const float cs = (float)s.cam->chunk_size * vs;
-  const i3 c = chunk_coord_from_pos(p, cs);
-  const uint32_t slot = grid_lookup_slot(s, c.x, c.y, c.z);
-  if (slot == INVALID || slot >= s.cam->chunk_count) return LeafQuery{p, vs, MAT_AIR};
-  const Meta ch = meta_at(s, slot);
-  const v3 rb = V3((float)ch.ox, (float)ch.oy, (float)ch.oz) * vs;
-  return query_leaf_at(s, p, rb, (float)s.cam->chunk_size * vs, ch.node_base, ch.macro_base);
-}
-
 // ---------------------------------------------------------------------------
 // wind.wgsl / leaves.wgsl
 // ---------------------------------------------------------------------------
@@ -744,8 +733,8 @@ __device__ __forceinline__ void st_release_gpu(uint32_t* p, uint32_t v) {
 }
 
 // Makes the record's lod-0 segment frames usable: ready already, or built
-// here by the first lane to claim them (the same grass_seg_frame values every
-// march would compute).  A lane that finds another one building them goes on
+// here by the first lane to claim them (the values every march would
+// compute).  A lane that finds another one building them goes on
 // without (false) and asks again at its next evaluation; nothing waits.
 __device__ __noinline__ bool grass_frames_ready(const Scene& s, GrassCellGeom& G) {
   uint32_t* st = s.grass_state + G.rec;
@@ -1552,7 +1541,7 @@ __device__ __forceinline__ v3 slab_task_corner(const uint4& a, const Meta& ch, v
 // Unsorted, the marches ran 8.8 of 32 lanes and half of L1's wavefronts.
 // With the normals taken for nearest hits only and the marches the walk left
 // open among the tasks: 1080p frame 4.34 -> 3.66 ms, the 64-request batch
-// 87 -> 63 ms (start 95), frame of lights 3.62 -> 3.34 ms, 256x144 frame
+// 87 -> 63 ms, frame of lights 3.62 -> 3.34 ms, 256x144 frame
 // 0.52 -> 0.53 ms.
 struct SlabSink {
   uint4* raw;          // tasks as found
@@ -2670,8 +2659,9 @@ __device__ __forceinline__ v3 sphere_dir_local(uint32_t i, uint32_t count) {  //
   return V3(cosf_(phi) * r, sinf_(phi) * r, y);
 }
 
-// query_leaf_world for the cell centres of a light ray: the material at p, and
-// for air the cube around p that is air throughout (size 0: none known).
+// The world leaf query (svo_query.wgsl:270-291) for the cell centres of a light
+// ray: the material at p, and for air the cube around p that is air throughout
+// (size 0: none known).
 __device__ __forceinline__ LeafQuery light_cell_query(const Scene& s, v3 p) {
   const float vs = vs_(s);
   const float cs = (float)s.cam->chunk_size * vs;

@@ -1782,10 +1782,8 @@ vxe_status build_launch(vxe_ctx* c, vxe::build::BuildArgs& B, uint32_t n) {
     vxe_status st = alloc(c, c->build_scratch, need);
     if (st != VXE_OK) return st;
   }
-  if (!c->build_ev[0]) {  // first build on this context: events, and the octree kernel's staging size
+  if (!c->build_ev[0])  // first build on this context
     for (auto& e : c->build_ev) CK(cudaEventCreate(&e));
-    CK(cudaFuncSetAttribute(vb::k_build_svo, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)vb::kStageBytes));
-  }
   B.cave_smin = cave_s_min((double)B.wp.cave_threshold);
   B.n = n;
   char* base = (char*)c->build_scratch.p;
@@ -1803,10 +1801,10 @@ vxe_status build_launch(vxe_ctx* c, vxe::build::BuildArgs& B, uint32_t n) {
   vb::k_build_columns<<<n * 16u, 256, 0, st>>>(B);
   CK(cudaGetLastError());
   CK(cudaEventRecord(c->build_ev[1], st));
-  vb::k_build_svo<<<n, vb::SVO_THREADS, vb::kStageBytes, st>>>(B);
+  vb::k_build_svo<<<n, vb::SVO_THREADS, 0, st>>>(B);
   CK(cudaGetLastError());
   if (B.place || B.node_cap) {  // a counting call writes no nodes
-    vb::k_build_ropes<<<n * vb::ROPE_PARTS, vb::ROPE_THREADS, 0, st>>>(B);
+    vb::k_build_voxels<<<n * vb::VOXEL_PARTS, vb::VOXEL_THREADS, 0, st>>>(B);
     CK(cudaGetLastError());
   }
   CK(cudaEventRecord(c->build_ev[2], st));

@@ -380,7 +380,8 @@ vxe_status vxe_view_destroy(vxe_ctx* ctx, vxe_view* view);
  * frame.  local_taa and composite_taa are fused into primary / composite and
  * report 0.  Extra fields (no reference counterpart): primary_trace is the
  * trace kernel inside `primary` (the rest of `primary` is shading) and
- * grass_cells the per-frame grass cell table, which `tiles` includes. */
+ * grass_cells the wait for the per-frame grass cell table where it is built
+ * ahead of the frame (`tiles` includes it); beside the walk it is in neither. */
 typedef struct vxe_timings {
   double primary, local_taa, godray, composite, composite_taa, tiles, total;
   /* extras: the trace stage of the wavefront schedule (walk, probe column

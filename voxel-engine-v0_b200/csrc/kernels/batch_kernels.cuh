@@ -503,7 +503,7 @@ __global__ void __launch_bounds__(BATCH_THREADS, SLAB_MIN_BLOCKS) k_batch_slab_e
   const uint32_t chunk = n >= warps * (SLAB_CHUNK / 2u) ? SLAB_CHUNK : 32u;  // few tasks: over all the warps
   for (uint32_t i = blockIdx.x * (BATCH_THREADS / 32) + (threadIdx.x >> 5); i * chunk < n; i += warps) {
     slab_march_chunk(
-        work[threadIdx.x >> 5], i * chunk, chunk, n,
+        work[threadIdx.x >> 5], B.grass_frames, i * chunk, chunk, n,
         [&](uint32_t j, SlabRay* r) {
           const BatchSlab w = batch_slab(B, n_reqs, j);
           *r = SlabRay{w.a, w.slot, w.ro, w.rd, w.id, w.cb};

@@ -1610,6 +1610,8 @@ __device__ __forceinline__ const float4* grass_column_frames(const Scene& s, uin
 // the chunk, and the survivors queue up again, so lanes whose march has ended
 // after one of up to seven evaluations do not wait for the longest (14.6 of
 // 32 lanes before).  The others march in place (grass_layer_march).
+//   frames           the launch's table (not a scene's: those of a batch's
+//                    requests with another wind have none)
 //   ray(j, &w)       task j's ray and cell; returns its scene
 //   done(j, hit, t)  its result, for every task of the chunk
 struct SlabRay {
@@ -1626,10 +1628,9 @@ struct SlabWarp {  // shared memory, one per warp
 };
 constexpr uint8_t SLAB_HIT = 254, SLAB_MISS = 255;
 template <class Ray, class Done>
-__device__ __forceinline__ void slab_march_chunk(SlabWarp& W, uint32_t base, uint32_t chunk, uint32_t n, Ray&& ray,
-                                                 Done&& done) {
+__device__ __forceinline__ void slab_march_chunk(SlabWarp& W, const float4* frames, uint32_t base, uint32_t chunk,
+                                                 uint32_t n, Ray&& ray, Done&& done) {
   const uint32_t lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
-  const float4* frames = nullptr;
   uint32_t tail = 0u;
   for (uint32_t r = 0; r < chunk; r += 32u) {
     const uint32_t k = r + lane, j = base + k;
@@ -1640,7 +1641,6 @@ __device__ __forceinline__ void slab_march_chunk(SlabWarp& W, uint32_t base, uin
       const float vs = vs_(s);
       const float t0 = __uint_as_float(w.a.z), t1 = __uint_as_float(w.a.w);
       const uint32_t lod = grass_lod_from_t(t0);
-      frames = s.grass_frames;
       const float4* F = lod == 0u ? grass_column_frames(s, w.slot, w.a.y & 4095u, w.cb, w.id) : nullptr;
       if (F == nullptr) {
         GrassCellGeom G;
@@ -1666,11 +1666,6 @@ __device__ __forceinline__ void slab_march_chunk(SlabWarp& W, uint32_t base, uin
     const uint32_t m = __ballot_sync(0xFFFFFFFFu, go);
     if (go) W.alive[tail + __popc(m & below)] = (uint8_t)k;
     tail += (uint32_t)__popc(m);
-  }
-  // (the scenes of a launch share the table: any lane's frames are all lanes')
-  for (uint32_t o = 16u; o; o >>= 1) {
-    const unsigned long long f = __shfl_xor_sync(0xFFFFFFFFu, (unsigned long long)(uintptr_t)frames, o);
-    if (frames == nullptr) frames = (const float4*)(uintptr_t)f;
   }
   __syncwarp();
   for (uint32_t head = 0u; head < tail;) {

@@ -1207,7 +1207,7 @@ __device__ __forceinline__ void k_slab_eval_body(const FrameArgs& A) {
   const uint32_t chunk = n >= warps * (SLAB_CHUNK / 2u) ? SLAB_CHUNK : 32u;  // few tasks: over all the warps
   for (uint32_t i = blockIdx.x * (SHADE_THREADS / 32) + (threadIdx.x >> 5); i * chunk < n; i += warps) {
     slab_march_chunk(
-        work[threadIdx.x >> 5], i * chunk, chunk, n,
+        work[threadIdx.x >> 5], A.grass_frames, i * chunk, chunk, n,
         [&](uint32_t j, SlabRay* r) -> const Scene& {
           const SlabWork w = slab_work(s, A, j);
           *r = SlabRay{w.a, w.slot, w.c.ro, w.c.rd, w.id, w.cb};

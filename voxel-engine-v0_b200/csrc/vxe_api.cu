@@ -89,7 +89,7 @@ struct FrameState {
   cudaGraph_t fgraph = nullptr;
   cudaGraphExec_t fgraph_exec = nullptr;
   std::vector<cudaGraphNode_t> fgraph_nodes;
-  uint64_t fgraph_key[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  uint64_t fgraph_key[9] = {};
   // set by launch_frame while an asynchronous read of the output image is in
   // flight: the composite (its writer) waits for it, the earlier passes do not
   cudaEvent_t composite_wait = nullptr;
@@ -913,10 +913,12 @@ vxe_status launch_frame_graph(vxe_ctx* c, FrameState& F, const vxe_camera_gpu& c
   bool use_grass = false;
   if ((rc = grass_table_acquire(c, st, reader, cam, &use_grass)) != VXE_OK) return rc;
   if (use_grass) grass_table_args(c, A);
-  const uint64_t key[8] = {F.iw, F.ih, F.pw, F.ph,
-                           (uint64_t)(c->flags & VXE_FLAG_PRIMARY_MEGAKERNEL) | (use_grass ? 2u : 0u) |
-                               (A.sun_map ? (uint64_t)cam.grid_dims[0] << 2 | (uint64_t)cam.grid_dims[2] << 34 : 0u),
+  // the sun horizon's launch shape in a word of its own (0: no horizon)
+  const uint64_t sun = A.sun_map ? (uint64_t)cam.grid_dims[0] << 32 | cam.grid_dims[2] : 0u;
+  const uint64_t key[9] = {F.iw, F.ih, F.pw, F.ph,
+                           (uint64_t)(c->flags & VXE_FLAG_PRIMARY_MEGAKERNEL) | (use_grass ? 2u : 0u), sun,
                            (uint64_t)c->shade_wave, (uint64_t)(uintptr_t)A.q_count, (uint64_t)(uintptr_t)A.px_first};
+  static_assert(sizeof key == sizeof F.fgraph_key && !(VXE_FLAG_PRIMARY_MEGAKERNEL & 2u), "one field per bit");
   if (!F.fgraph_exec || std::memcmp(key, F.fgraph_key, sizeof key) != 0) {
     if (F.fgraph_exec) cudaGraphExecDestroy(F.fgraph_exec);
     if (F.fgraph) cudaGraphDestroy(F.fgraph);

@@ -1,0 +1,53 @@
+"""Sun horizons of large grids: a context of any grid capacity can be made, and
+frames of grids around the largest that has a horizon equal the oracle's.  A
+few chunks stand in a wide, otherwise empty grid.  Tolerance 0."""
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+from parity import compare_frame, make_renderer, read_gpu_frame
+from vxe import _abi as A
+from vxe.renderer import Renderer
+from vxe.scenes import FrameDriver, Scene
+from vxe.world import WorldSpec
+
+pytestmark = pytest.mark.gpu
+
+
+def test_grid_capacity_beyond_any_horizon():
+    # 2^27 cells (0.5 GB); a horizon for as many columns would take 275 GB
+    r = Renderer(8, 8, 1.0, node_capacity=64, chunk_capacity=1, grid_capacity=1 << 27, clip_levels=1, clip_res=16)
+    r.close()
+
+
+@pytest.mark.parametrize("dims,at", [((128, 1, 128), (126, 0, 126)), ((129, 1, 128), (60, 0, 60)),
+                                     ((16384, 1, 1), (9000, 0, 0)), ((1, 1, 16385), (0, 0, 9000)),
+                                     ((3, 300, 3), (0, 2, 0)), ((2, 700, 2), (0, 620, 0)), ((100, 3, 70), (0, 1, 33))])
+def test_frames_of_wide_grids_bit_exact(dims, at):
+    spec = WorldSpec(seed=4242, height_min=10, height_max=40, dirt_depth=3, carve_mod=50, cave_threshold=0.6,
+                     height_scale_vox=48.0, features=1)
+    inner = tuple(min(2, d) for d in (dims[0], 1, dims[2]))
+    path = lambda f: (np.array([3.2 * inner[0], 5.2, 1.5]) + 0.07 * f, 0.5, -0.25)  # noqa: E731
+    sc = Scene("wide", spec, (0, 0, 0), inner, (97, 61), 1.0, 3, 128, 2, node_capacity=1 << 20, path=path)
+    drv = FrameDriver(sc)
+    ups = drv.initial_uploads()
+    w = drv.world
+    grid = np.full(dims[::-1], A.INVALID_U32, dtype=np.uint32)
+    grid[at[2]:at[2] + inner[2], at[1]:at[1] + 1, at[0]:at[0] + inner[0]] = w.grid.reshape(inner[::-1])
+    w.grid, w.grid_dims, w.grid_capacity = grid.reshape(-1), dims, grid.size
+    w.grid_origin = tuple(-a for a in at)
+    r = make_renderer(sc, w)
+    try:
+        r.upload_world(w, ups)
+        ora = O.OracleFrameRunner(w, sc.internal, sc.present, drv.clip.tex, sc.clip_res, godray_alias=True)
+        for _ in range(2):
+            _, _, (params, patches), cam = drv.step()
+            r.write_clipmap_updates(params, patches)
+            r.write_camera(cam)
+            r.encode_compute()
+            ora.render(cam, params)
+            bad = compare_frame(read_gpu_frame(r), ora.outputs())
+            assert bad == {}, bad
+        assert r.read_error_word() == 0
+    finally:
+        r.close()

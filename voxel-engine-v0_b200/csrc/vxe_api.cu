@@ -438,10 +438,15 @@ void fill_scene_args(const vxe_ctx* c, FrameArgs& A) {
   A.slot_cells = (const uint8_t*)c->slot_cells.p;
 }
 
+// Grids of more chunk columns march every sun ray: a column takes 2 KB of a
+// horizon, so these (819 m square) take 34 MB per context and lane whatever the
+// grid capacity is.
+constexpr uint32_t kSunColumnsMax = 128u * 128u;
+
 // Bytes of one sun horizon (FrameArgs::sun_map): a grid has at most
 // grid_capacity chunk columns.
 size_t sun_bytes(const vxe_ctx* c) {
-  return (size_t)c->cfg.grid_capacity * (2u * vxe::dev::SUN_CELLS * vxe::dev::SUN_CELLS + 1u) * 4u;
+  return (size_t)std::min(c->cfg.grid_capacity, kSunColumnsMax) * (2u * vxe::dev::SUN_CELLS * vxe::dev::SUN_CELLS + 1u) * 4u;
 }
 
 // The horizon of the frame `A` on stream `st`, into A.sun_map (null: none).
@@ -451,10 +456,10 @@ void sun_enqueue(const FrameArgs& A, cudaStream_t st) {
   vxe::dev::k_sun_tops<<<dim3(nx, nz), vxe::dev::SUN_THREADS, 0, st>>>(A);
   vxe::dev::k_sun_horizon<<<dim3(nx, nz), vxe::dev::SUN_THREADS, 0, st>>>(A);
 }
-// A grid that a horizon can be made for (a launch has at most 65535 rows).
+// A grid that a horizon is made for.
 bool sun_usable(const vxe_camera_gpu& cam) {
   return cam.chunk_count != 0 && cam.grid_dims[0] != 0 && cam.grid_dims[1] != 0 && cam.grid_dims[2] != 0 &&
-         cam.grid_dims[2] <= 65535u;
+         (uint64_t)cam.grid_dims[0] * cam.grid_dims[2] <= kSunColumnsMax;  // (a launch has at most 65535 rows)
 }
 
 // Recomputes the light flags of slots [first, first + n) on the upload

@@ -322,24 +322,40 @@ constexpr int SUN_THREADS = (int)(SUN_CELLS * SUN_CELLS);
 
 // The cell tops: world height (voxels) of the highest non-air leaf over each
 // cell.  A slot whose meta does not stand in its grid cell bars the shortcut
-// for its column.
+// for its column.  The column's slots are looked up by one thread each, ahead
+// of the cells: one after another they were two dependent loads per slot (a
+// grid 64 chunks high held a 16x9 frame back by 0.15 ms).
 __global__ void __launch_bounds__(SUN_THREADS) k_sun_tops(const __grid_constant__ FrameArgs A) {
   __shared__ float red[SUN_THREADS / 32];
+  __shared__ uint32_t slot_s[SUN_THREADS];
+  __shared__ int32_t oy_s[SUN_THREADS];
   const Scene s = make_scene(A, false);
   const uint32_t nx = A.cam.grid_dims[0], ny = A.cam.grid_dims[1], nz = A.cam.grid_dims[2];
   const uint32_t ix = blockIdx.x, iz = blockIdx.y, t = threadIdx.x;
   float top = -BIG;
-  for (uint32_t iy = 0; iy < ny; ++iy) {
-    const uint32_t slot = grid_at(s, (iz * ny + iy) * nx + ix);
-    if (slot == INVALID || slot >= A.cam.chunk_count) continue;
-    const Meta m = meta_at(s, slot);
-    if (m.ox != (A.cam.grid_origin_chunk[0] + (int32_t)ix) * 64 || m.oy != (A.cam.grid_origin_chunk[1] + (int32_t)iy) * 64 ||
-        m.oz != (A.cam.grid_origin_chunk[2] + (int32_t)iz) * 64 || slot >= A.metas_n) {
-      top = BIG;
-      continue;
+  for (uint32_t iy0 = 0; iy0 < ny; iy0 += SUN_THREADS) {
+    const uint32_t m = min(ny - iy0, (uint32_t)SUN_THREADS);
+    bool barred = false;
+    if (t < m) {
+      uint32_t slot = grid_at(s, (iz * ny + iy0 + t) * nx + ix);
+      if (slot != INVALID && slot >= A.cam.chunk_count) slot = INVALID;
+      if (slot != INVALID) {
+        const Meta c = meta_at(s, slot);
+        barred = c.ox != (A.cam.grid_origin_chunk[0] + (int32_t)ix) * 64 ||
+                 c.oy != (A.cam.grid_origin_chunk[1] + (int32_t)(iy0 + t)) * 64 ||
+                 c.oz != (A.cam.grid_origin_chunk[2] + (int32_t)iz) * 64 || slot >= A.metas_n;
+        if (barred) slot = INVALID;
+        oy_s[t] = c.oy;
+      }
+      slot_s[t] = slot;
     }
-    const uint32_t h = A.slot_cells[(size_t)slot * SUN_THREADS + t];
-    if (h != 0u) top = fmax_(top, (float)(m.oy + (int32_t)h));
+    if (__syncthreads_or(barred)) top = BIG;
+    for (uint32_t j = 0; j < m; ++j) {
+      if (slot_s[j] == INVALID) continue;
+      const uint32_t h = A.slot_cells[(size_t)slot_s[j] * SUN_THREADS + t];
+      if (h != 0u) top = fmax_(top, (float)(oy_s[j] + (int32_t)h));
+    }
+    __syncthreads();
   }
   const uint32_t cells = nx * nz * SUN_THREADS;
   A.sun_map[cells + (iz * SUN_CELLS + t / SUN_CELLS) * (nx * SUN_CELLS) + ix * SUN_CELLS + t % SUN_CELLS] = top;
@@ -356,31 +372,32 @@ __global__ void __launch_bounds__(SUN_THREADS) k_sun_tops(const __grid_constant_
 // start in it, less what they have risen on reaching it.  Such rays move
 // equally in +x and +z, so k cells on they cross only the cells (k, k),
 // (k + 1, k) and (k, k + 1), having gone more than k - 1 (the first) or k
-// (the others) cells along each axis.
+// (the others) cells along each axis.  A horizon is at least the grid's
+// bottom, which ends the search over empty columns after the grid's height.
 __global__ void __launch_bounds__(SUN_THREADS) k_sun_horizon(const __grid_constant__ FrameArgs A) {
   const uint32_t nx = A.cam.grid_dims[0], nz = A.cam.grid_dims[2];
   const uint32_t w = nx * SUN_CELLS, hgt = nz * SUN_CELLS, cells = w * hgt;
   const float* top = A.sun_map + cells;
   const float* col_top = top + cells;
   // no cell of this column's rays is higher than the chunk columns they cross
-  __shared__ float bound_s;
-  if (threadIdx.x == 0u) {
-    float b = -BIG;
-    for (uint32_t k = 0; blockIdx.x + k < nx && blockIdx.y + k < nz; ++k) {
-      const uint32_t x = blockIdx.x + k, z = blockIdx.y + k;
-      b = fmax_(b, col_top[z * nx + x]);
-      if (x + 1u < nx) b = fmax_(b, col_top[z * nx + x + 1u]);
-      if (z + 1u < nz) b = fmax_(b, col_top[(z + 1u) * nx + x]);
-    }
-    bound_s = b;
+  float b = -BIG;
+  for (uint32_t k = threadIdx.x; blockIdx.x + k < nx && blockIdx.y + k < nz; k += SUN_THREADS) {
+    const uint32_t x = blockIdx.x + k, z = blockIdx.y + k;
+    b = fmax_(b, col_top[z * nx + x]);
+    if (x + 1u < nx) b = fmax_(b, col_top[z * nx + x + 1u]);
+    if (z + 1u < nz) b = fmax_(b, col_top[(z + 1u) * nx + x]);
   }
+  __shared__ float red[SUN_THREADS / 32];
+  for (int o = 16; o; o >>= 1) b = fmax_(b, __shfl_xor_sync(0xFFFFFFFFu, b, o));
+  if ((threadIdx.x & 31u) == 0u) red[threadIdx.x >> 5] = b;
   __syncthreads();
-  const float bound = bound_s;
+  float bound = red[0];
+  for (int k = 1; k < SUN_THREADS / 32; ++k) bound = fmax_(bound, red[k]);
   const uint32_t x0 = blockIdx.x * SUN_CELLS + threadIdx.x % SUN_CELLS, z0 = blockIdx.y * SUN_CELLS + threadIdx.x / SUN_CELLS;
   // height gained per cell, rounded down
   const float rise = (float)SUN_CELL_VOX * (SUN_Y / SUN_X) * 0.9999f;
   static_assert(SUN_X == SUN_Z && SUN_X > 0.0f && SUN_Y > 0.0f, "the sun's rays run along the diagonal and rise");
-  float h = -BIG;
+  float h = bound < BIG ? (float)(A.cam.grid_origin_chunk[1] * 64) : BIG;  // a barred column ahead bars its rays
   for (uint32_t k = 0; x0 + k < w && z0 + k < hgt; ++k) {
     const float near = k == 0u ? 0.0f : rise * (float)(k - 1u), far = rise * (float)k;
     if (bound - near <= h) break;

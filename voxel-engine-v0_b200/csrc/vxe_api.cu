@@ -440,7 +440,8 @@ void fill_scene_args(const vxe_ctx* c, FrameArgs& A) {
 
 // Grids of more chunk columns march every sun ray: a column takes 2 KB of a
 // horizon, so these (819 m square) take 34 MB per context and lane whatever the
-// grid capacity is.
+// grid capacity is.  At this many a frame is still faster with the horizon than
+// without: 64x36 0.92 against 1.00 ms, 256x144 1.10 / 1.13, 960x540 2.67 / 2.85.
 constexpr uint32_t kSunColumnsMax = 128u * 128u;
 
 // Bytes of one sun horizon (FrameArgs::sun_map): a grid has at most

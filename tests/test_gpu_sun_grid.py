@@ -5,11 +5,11 @@ import numpy as np
 import pytest
 
 from oracle import oracle as O
-from parity import compare_frame, make_renderer, read_gpu_frame
+from parity import compare_frame, make_renderer, read_gpu_frame, run_parity
 from vxe import _abi as A
 from vxe.renderer import Renderer
 from vxe.scenes import FrameDriver, Scene
-from vxe.world import WorldSpec
+from vxe.world import WorldSpec, ground_height
 
 pytestmark = pytest.mark.gpu
 
@@ -51,3 +51,18 @@ def test_frames_of_wide_grids_bit_exact(dims, at):
         assert r.read_error_word() == 0
     finally:
         r.close()
+
+
+@pytest.mark.parametrize("ox,oz,k", [(33000, 0, 2), (70000, 0, 0), (130000, 0, 6), (-130000, -130000, 3),
+                                     (250000, 0, 6), (-250000, -250000, 3)])
+def test_far_from_the_origin_bit_exact(ox, oz, k):
+    # where binary32 positions are cells apart, a point's own cell is among those read or the ray marches
+    spec = WorldSpec(seed=100 + k, height_min=5, height_max=60, dirt_depth=3, carve_mod=(0, 50)[k % 2],
+                     cave_threshold=(0.6, 0.5, 2.0)[k % 3], height_scale_vox=(4.0, 8.0, 16.0, 48.0)[k % 4], features=1 + k % 3)
+    ox, oz = ox + k, oz + (k if oz else 0)
+    at = np.array([ox * 6.4 + 2.0 + k * 0.3, 0.0, oz * 6.4 + 2.0])
+    at[1] = 0.1 * ground_height(spec, int(at[0] * 10), int(at[2] * 10)) + (1.0, 2.0, 4.0, 0.5)[k % 4]
+    sc = Scene("far", spec, (ox, 0, oz), (3, 1, 3), (97, 61), 1.0, 3, 128, 2, node_capacity=1 << 20,
+               path=lambda f: (at + 0.5 * f, 0.7 + k, -0.25 - 0.1 * (k % 3)))
+    res = run_parity(sc, frames=2)
+    assert all(r == {} for r in res), res

@@ -2563,6 +2563,7 @@ __device__ __forceinline__ bool sun_clear(const Scene& s, v3 p, bool* barred) {
   if (!(x0 >= 0.0f && z0 >= 0.0f && x1 < nx && z1 < nz)) return false;  // outside the grid, or NaN
   const uint32_t w = s.cam->grid_dims[0] * SUN_CELLS;
   const uint32_t i0 = (uint32_t)x0, i1 = (uint32_t)x1, j0 = (uint32_t)z0, j1 = (uint32_t)z1;
+  if (i1 - i0 > 2u || j1 - j0 > 2u) return false;  // beyond 4e6 voxels: cells between that these do not cover
   float h = __ldg(&s.sun_map[j0 * w + i0]);
   if (i1 != i0 || j1 != j0)
     h = fmax_(fmax_(h, __ldg(&s.sun_map[j0 * w + i1])), fmax_(__ldg(&s.sun_map[j1 * w + i0]), __ldg(&s.sun_map[j1 * w + i1])));

@@ -2660,7 +2660,8 @@ __device__ __forceinline__ v3 sphere_dir_local(uint32_t i, uint32_t count) {  //
 
 // The world leaf query (svo_query.wgsl:270-291) for the cell centres of a light
 // ray: the material at p, and for air the cube around p that is air throughout
-// (size 0: none known).
+// (size 0: none known, as where the slot's meta stands elsewhere than the grid
+// cell it serves: its cubes are then not this cell's alone).
 __device__ __forceinline__ LeafQuery light_cell_query(const Scene& s, v3 p) {
   const float vs = vs_(s);
   const float cs = (float)s.cam->chunk_size * vs;
@@ -2669,6 +2670,9 @@ __device__ __forceinline__ LeafQuery light_cell_query(const Scene& s, v3 p) {
   const uint32_t slot = grid_lookup_slot(s, c.x, c.y, c.z);
   if (slot == INVALID || slot >= s.cam->chunk_count) return air;
   const Meta ch = meta_at(s, slot);
+  const int32_t csv = (int32_t)s.cam->chunk_size;
+  const bool home = ch.ox == c.x * csv && ch.oy == c.y * csv && ch.oz == c.z * csv;
+  auto leaf = [home](v3 b, float sz, uint32_t mat) { return LeafQuery{b, home ? sz : 0.0f, mat}; };
   const v3 rb = V3((float)ch.ox, (float)ch.oy, (float)ch.oz) * vs;
   if (ch.macro_base != INVALID) {
     const float cell = macro_cell_size(cs);
@@ -2678,22 +2682,22 @@ __device__ __forceinline__ LeafQuery light_cell_query(const Scene& s, v3 p) {
     if (mx < 0 || my < 0 || mz < 0 || mx >= (int32_t)MACRO_DIM || my >= (int32_t)MACRO_DIM || mz >= (int32_t)MACRO_DIM)
       return air;
     if (!macro_test(s, ch.macro_base, macro_bit_index((uint32_t)mx, (uint32_t)my, (uint32_t)mz)))
-      return LeafQuery{rb + V3((float)mx, (float)my, (float)mz) * cell, cell, MAT_AIR};
+      return leaf(rb + V3((float)mx, (float)my, (float)mz) * cell, cell, MAT_AIR);
   }
   uint32_t idx = ch.node_base;
   v3 bmin = rb;
   float size = cs;
   for (uint32_t d = 0; d < 32; ++d) {
     const Node n = node_global(s, idx);
-    if (n.child_base == LEAF) return LeafQuery{bmin, size, n.material};
-    if (d >= chunk_max_depth(s)) return LeafQuery{bmin, size, MAT_AIR};
+    if (n.child_base == LEAF) return leaf(bmin, size, n.material);
+    if (d >= chunk_max_depth(s)) return leaf(bmin, size, MAT_AIR);
     const float half = size * 0.5f;
     const v3 mid = bmin + V3s(half);
     const float e = 1e-6f * size;
     const uint32_t hx = p.x > mid.x + e ? 1u : 0u, hy = p.y > mid.y + e ? 1u : 0u, hz = p.z > mid.z + e ? 1u : 0u;
     const uint32_t ci = hx | (hy << 1) | (hz << 2);
     const v3 cb = bmin + V3(hx ? half : 0.0f, hy ? half : 0.0f, hz ? half : 0.0f);
-    if ((n.child_mask & (1u << ci)) == 0u) return LeafQuery{cb, half, MAT_AIR};
+    if ((n.child_mask & (1u << ci)) == 0u) return leaf(cb, half, MAT_AIR);
     idx = ch.node_base + (n.child_base + child_rank(n.child_mask, ci));
     bmin = cb;
     size = half;

@@ -2009,6 +2009,9 @@ constexpr size_t kStageHdr = 0, kStageReqs = 64,
 // Stored probes and slab tasks per viewport ray of a batch; rays past the
 // budget walk again with inline probes.
 constexpr uint32_t kBatchProbesPerRay = 4, kBatchSlabsPerRay = 2;
+// Most viewport rays of a persistent or graph batch: as many as there are 30-bit
+// probe records for (100 GB of lane buffers).
+constexpr uint32_t kBatchRaysMax = 0x3FFFFFFFu / kBatchProbesPerRay;
 // Slab bins of a batch (SlabSink::bits): its viewports stand all over the world.
 constexpr uint32_t kBatchSlabBits = 6;
 constexpr size_t kBatchCountBytes = 64 + (size_t)(4096u << (kBatchSlabBits + 1u)) * 4;
@@ -2040,8 +2043,7 @@ vxe_status lane_resources(vxe_ctx* c, BatchLane& L, uint32_t tiles, uint32_t vp_
     c->b_tile_grid = sms * std::max(lb, 1);
   }
   if (vp_rays > L.ray_cap) {
-    const uint64_t cap = std::min<uint64_t>(std::max<uint64_t>((uint64_t)vp_rays + vp_rays / 2, 1u << 16),
-                                            0x3FFFFFFFu / kBatchProbesPerRay);
+    const uint64_t cap = std::min<uint64_t>(std::max<uint64_t>((uint64_t)vp_rays + vp_rays / 2, 1u << 16), kBatchRaysMax);
     if ((st = alloc_on(c, L.px_first, cap * 8, L.stream)) != VXE_OK) return st;
     if ((st = alloc_on(c, L.px_mask, cap * 8, L.stream)) != VXE_OK) return st;
     if ((st = alloc_on(c, L.px_probe, cap * 8, L.stream)) != VXE_OK) return st;
@@ -2253,6 +2255,8 @@ vxe_status vxe_submit_batch_async(vxe_ctx* c, uint32_t lane, const vxe_request* 
   // is the per-request single-launch baseline with the reference's inline
   // probes.
   const bool defer = opt->mode != VXE_BATCH_PLAIN && vp_rays != 0;
+  if (defer && vp_rays > kBatchRaysMax)
+    return fail(c, VXE_ERR_CAPACITY, "persistent batch of more than %u viewport rays", kBatchRaysMax);
   const uint32_t vp_items = items;
   if (sorted) items += (uint32_t)((q_rays + 128u * rpt - 1) / (128u * rpt));
   vxe_status st = lane_resources(c, L, tiles, defer ? (uint32_t)vp_rays : 0u, sorted ? (uint32_t)q_rays : 0u);

@@ -40,7 +40,7 @@ struct BatchReq {  // 80 B
 struct BatchHeader {
   uint32_t n_reqs, total_tiles, n_items, tile_w, tile_h, rpt, tile_reqs, vp_rays;
   // coherent queries (k_batch_queries): rays in sorted order, q_unit per warp
-  uint32_t vp_items, q_rays, nbins, sorted, q_unit;
+  uint32_t vp_items, q_rays, nbins, q_unit;
 };
 
 struct BatchArgs {

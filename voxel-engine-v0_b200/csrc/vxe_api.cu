@@ -2206,7 +2206,8 @@ vxe_status vxe_submit_batch_async(vxe_ctx* c, uint32_t lane, const vxe_request* 
   uint32_t tiles = 0, items = 0;
   uint64_t rays = 0, vp_rays = 0, q_rays = 0;
   // Coherent queries (persistent and graph modes): query rays are traced in
-  // bin order after every viewport item instead of as per-request items.
+  // bin order beside the viewport items (k_batch_queries) instead of as
+  // per-request items.
   bool sorted = false;
   if (opt->mode != VXE_BATCH_PLAIN)
     for (uint32_t i = 0; i < n; ++i) sorted = sorted || reqs[i].kind == VXE_REQ_QUERY;
@@ -2258,12 +2259,13 @@ vxe_status vxe_submit_batch_async(vxe_ctx* c, uint32_t lane, const vxe_request* 
   if (defer && vp_rays > kBatchRaysMax)
     return fail(c, VXE_ERR_CAPACITY, "persistent batch of more than %u viewport rays", kBatchRaysMax);
   const uint32_t vp_items = items;
+  // (queries taken in bin order are no items; the statistics count them in the options' units all the same)
   if (sorted) items += (uint32_t)((q_rays + 128u * rpt - 1) / (128u * rpt));
   vxe_status st = lane_resources(c, L, tiles, defer ? (uint32_t)vp_rays : 0u, sorted ? (uint32_t)q_rays : 0u);
   if (st != VXE_OK) return st;
   if (c->upload_recorded) CK(cudaStreamWaitEvent(L.stream, c->upload_done, 0));
   const uint32_t nbins = std::max(c->cfg.grid_capacity, 1u) * 8u;
-  BatchHeader H{n, tiles, items, tw, th, rpt, n, (uint32_t)vp_rays, vp_items, (uint32_t)q_rays, nbins, sorted ? 1u : 0u,
+  BatchHeader H{n, tiles, items, tw, th, rpt, n, (uint32_t)vp_rays, vp_items, (uint32_t)q_rays, nbins,
                 query_unit(q_rays, (uint32_t)c->b_query_grid * (BATCH_THREADS / 32))};
   std::memcpy((char*)L.stage + kStageHdr, &H, sizeof H);
   if (n) std::memcpy((char*)L.stage + kStageReqs, R.data(), n * sizeof(BatchReq));

@@ -1465,7 +1465,7 @@ __device__ __forceinline__ HitGeom make_hit(uint32_t mat, float t, v3 n, v3 rb, 
 //   k_probe_dda   runs each stored probe's column DDA, one lane each, and
 //                 stores one task per grass slab it meets;
 //   k_slab_bases, k_slab_order   sort the tasks by lod and cell;
-//   k_slab_eval   marches every slab, one lane each;
+//   k_slab_eval   marches every slab, a warp's chunk of tasks in turns;
 //   resolve       rebuilds the candidate loop's answer from the parts.
 // Why the parts suffice: the candidate loop keeps the nearest chunk result
 // (earliest chunk on ties) and a chunk's result is its first probe hit, else

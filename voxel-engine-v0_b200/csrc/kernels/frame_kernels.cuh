@@ -1213,7 +1213,7 @@ __device__ __forceinline__ SlabWork slab_work(const Scene& s, const FrameArgs& A
   return w;
 }
 
-// One lane per grass slab: the blade march of try_grass_slab_hit.  A hit
+// The blade march of try_grass_slab_hit for every grass slab (slab_march_chunk).  A hit
 // lowers its pixel's nearest-hit key and marks its chunk; k_slab_pick takes
 // the normals, of the nearest hits only (13 % of the marches hit, and their
 // normals inside this kernel cost every warp about two more marches).
@@ -1658,7 +1658,7 @@ __device__ __forceinline__ void k_shade_vox_body(const FrameArgs& A) {
     }
     const PrimaryCtx c = primary_ctx(s, pix % A.iw, pix / A.iw, A.iw);
     const uint4* src = A.pix_hit + (size_t)pix * 5u;
-    const HitGeom g = load_pixhit(s, src);  // t and n as refined by k_shade_prep
+    const HitGeom g = load_pixhit(s, src);  // t and n as k_shade_refine or k_primary_walk left them
     const uint4 e = src[3], f = src[4];
     const float shadow_out = shadow_fresh(c) ? shadow_blend(s, A, c, c.ro + c.rd * g.t, A.px_shadow[pix])
                                              : clampf(A.shadow_in[c.pix], 0.0f, 1.0f);

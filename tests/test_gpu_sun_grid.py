@@ -20,6 +20,16 @@ def test_grid_capacity_beyond_any_horizon():
     r.close()
 
 
+def test_lane_bytes_count_the_horizon():
+    sizes = []
+    for cells in (1, 1000, 128 * 128, 128 * 128 + 1):
+        r = Renderer(8, 8, 1.0, node_capacity=64, chunk_capacity=1, grid_capacity=cells, clip_levels=1, clip_res=16)
+        sizes.append(r.view_lane_bytes(64, 36, 1.0))
+        r.close()
+    column = 2 * 16 * 16 * 4 + 4  # horizon and tops of 16 x 16 cells, their maximum
+    assert [s - sizes[0] for s in sizes[1:]] == [999 * column, 16383 * column, 16383 * column]
+
+
 @pytest.mark.parametrize("dims,at", [((128, 1, 128), (126, 0, 126)), ((129, 1, 128), (60, 0, 60)),
                                      ((16384, 1, 1), (9000, 0, 0)), ((1, 1, 16385), (0, 0, 9000)),
                                      ((3, 300, 3), (0, 2, 0)), ((2, 700, 2), (0, 620, 0)), ((100, 3, 70), (0, 1, 33))])

@@ -2428,7 +2428,7 @@ uint64_t vxe_view_lane_bytes(const vxe_ctx* c, uint32_t present_w, uint32_t pres
   if (!c || present_w == 0 || present_h == 0 || !(render_scale > 0.0f)) return 0;
   FrameState F;
   set_dims(F, present_w, present_h, render_scale);
-  uint64_t total = 0;
+  uint64_t total = sun_bytes(c);
   for (int i = 0; i < IMG_N; ++i)
     if (img_enabled(c, i) && img_is_scratch(i)) total += img_bytes(F, i);
   return total;

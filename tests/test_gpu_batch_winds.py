@@ -96,3 +96,27 @@ def test_wide_batch_reaches_the_wide_chunks(scene):
         tasks += r.frame_stats()["slab_tasks"]
     r.resize_output(64, 36)
     assert tasks > _wide_tasks() + 64, tasks
+
+
+@pytest.mark.parametrize("first,other", [(0.1, 0.05), (0.12, 0.1)])
+def test_voxel_sizes_in_one_batch_match_cold_frames(scene, first, other):
+    # the table holds cells of the first viewport's voxel size only
+    torch, sc, w, r = scene
+    reqs, outs = _requests(torch, sc, w, [(0, 160, 90, 0.0, 1.0), (0, 160, 90, 0.0, 1.0), (24, 97, 61, 0.0, 1.0)])
+    for q, vs in zip(reqs, (first, other, other)):
+        q.camera.voxel_params[0] = vs
+    r.set_flags(r.flags | A.FLAG_HIT_RECORDS)
+    want = []
+    for q in reqs:
+        r.resize_output(q.width, q.height)
+        r.write_camera(q.camera)
+        r.encode_compute()
+        want.append(r.read_image(A.IMG_HITS).tobytes())
+    r.resize_output(64, 36)
+    r.set_flags(r.flags & ~A.FLAG_HIT_RECORDS)
+    for mode in (A.BATCH_PLAIN, A.BATCH_PERSISTENT, A.BATCH_GRAPH, A.BATCH_GRAPH):
+        r.submit_batch(reqs, (8, 4), 1, mode)
+        for i, (o, x) in enumerate(zip(outs, want)):
+            assert o.cpu().numpy().tobytes() == x, (mode, i)
+            o.zero_()
+        torch.cuda.synchronize()

@@ -121,7 +121,7 @@ struct BatchLane {
   uint32_t q_cap = 0;
   void* stage = nullptr;  // pinned: header | requests | cameras
   cudaGraphExec_t graph = nullptr;
-  uint32_t graph_key[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+  uint32_t graph_key[10] = {};
   vxe_clipmap_gpu graph_clip{};  // clipmap uniform baked into the captured launches
   cudaEvent_t ev[2] = {nullptr, nullptr};
   bool busy = false;
@@ -2288,7 +2288,7 @@ vxe_status vxe_submit_batch_async(vxe_ctx* c, uint32_t lane, const vxe_request* 
   if (defer && sorted && (st = side_ready(c, L.side)) != VXE_OK) return st;  // created outside a capture
   CK(cudaEventRecord(L.ev[0], L.stream));
   // Grass cell table for the wind of the first viewport's camera (requests
-  // with another wind time / strength derive their cells in the march).
+  // with another wind time / strength or voxel size derive their cells in the march).
   const vxe_camera_gpu* gcam = &cams[0];
   for (uint32_t i = 0; i < n; ++i)
     if (reqs[i].kind == VXE_REQ_VIEWPORT) {
@@ -2305,6 +2305,7 @@ vxe_status vxe_submit_batch_async(vxe_ctx* c, uint32_t lane, const vxe_request* 
     B.grass_taper = (const float*)c->gt.taper.p;
     B.grass_time_bits = fbits(gcam->voxel_params[1]);
     B.grass_strength_bits = fbits(gcam->voxel_params[2]);
+    B.grass_vs_bits = fbits(gcam->voxel_params[0]);
   }
   if (opt->mode == VXE_BATCH_PLAIN) {
     CK(cudaMemcpyAsync(L.hdr.p, (char*)L.stage + kStageHdr, sizeof H, cudaMemcpyHostToDevice, L.stream));
@@ -2326,10 +2327,11 @@ vxe_status vxe_submit_batch_async(vxe_ctx* c, uint32_t lane, const vxe_request* 
   } else {
     // Captured once per tile-buffer allocation and clipmap uniform; later
     // batches only rewrite the pinned staging the graph's copies read.
-    const uint32_t key[9] = {(uint32_t)(uintptr_t)L.tile_count.p, (uint32_t)((uintptr_t)L.tile_count.p >> 32),
-                             (uint32_t)c->cfg.clip_levels, c->clip.levels, c->clip.res, 1u,
-                             (use_grass ? 1u : 0u) | (B.defer ? 2u : 0u) | (sorted ? 4u : 0u), B.grass_time_bits,
-                             B.grass_strength_bits};
+    const uint32_t key[10] = {(uint32_t)(uintptr_t)L.tile_count.p, (uint32_t)((uintptr_t)L.tile_count.p >> 32),
+                              (uint32_t)c->cfg.clip_levels, c->clip.levels, c->clip.res, 1u,
+                              (use_grass ? 1u : 0u) | (B.defer ? 2u : 0u) | (sorted ? 4u : 0u), B.grass_time_bits,
+                              B.grass_strength_bits, B.grass_vs_bits};
+    static_assert(sizeof key == sizeof L.graph_key, "one word per field");
     const bool same = L.graph != nullptr && std::memcmp(key, L.graph_key, sizeof key) == 0 &&
                       std::memcmp(&L.graph_clip, &B.clip, sizeof B.clip) == 0;
     if (!same) {

@@ -319,7 +319,8 @@ typedef struct vxe_batch_stats {
 #define VXE_MAX_BATCH_REQUESTS 256u
 #define VXE_BATCH_LANES 4u
 /* Traces n (<= VXE_MAX_BATCH_REQUESTS) requests; returns when they are done
- * (lane 0). */
+ * (lane 0).  A persistent or graph batch has less than 2^28 viewport rays, any
+ * batch less than 2^30 and less than 2^30 query rays (VXE_ERR_CAPACITY). */
 vxe_status vxe_submit_batch(vxe_ctx* ctx, const vxe_request* reqs, uint32_t n, const vxe_batch_options* opt,
                             vxe_batch_stats* stats);
 /* Asynchronous form: each of the VXE_BATCH_LANES lanes owns a stream, staging
